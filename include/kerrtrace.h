@@ -60,7 +60,7 @@ typedef enum kt_precision { KT_PREC_FP32 = 0, KT_PREC_MIXED = 1, KT_PREC_FP64 = 
 /* Scheduling of the trace kernel.  All schedules produce the same image bits. */
 typedef enum kt_schedule {
     KT_SCHED_PLAIN = 0,     /* one thread per pixel on a 2D grid of block_dim tiles (kernel.cu:88) */
-    KT_SCHED_WAVEFRONT = 1, /* persistent kernel, lanes refilled from a device work counter */
+    KT_SCHED_WAVEFRONT = 1, /* persistent kernel, warps take units of 32 rays from a work counter */
     KT_SCHED_AUTO = 2       /* whichever the context's kt_tuning selects (the autotuner's choice) */
 } kt_schedule;
 
@@ -80,7 +80,8 @@ typedef struct kt_tuning {
     int32_t blocks_per_sm; /* wavefront: resident blocks of 128 threads per SM, 3..6; plain (blocks
                               of at most 128 threads): 5 or 6 (FP32, mixed) or 3 or 4 (FP64) asks
                               for that many resident blocks, anything else for the default shape */
-    int32_t refill_min;    /* wavefront: idle lanes a warp collects before refilling them, 1..32 */
+    int32_t refill_min;    /* 1..32; kept for its callers, without effect: a warp of the wavefront
+                              schedule takes its next rays when all 32 lanes are idle */
     int32_t order;         /* kt_order; KT_ORDER_LONG_FIRST allocates a 4-byte-per-pixel buffer */
     int32_t keep_frozen;   /* 0 (default): a ray whose state has become NaN (the reference's
                               tolerance reaches 0 near the hole, cuda/kerr_trace.cuh:66-73) is
@@ -260,8 +261,7 @@ kt_status kt_trace_progressive(kt_context* ctx, void* stream, const kt_camera* c
                                uint32_t n_samples, float* accum, float* hdr_out, uint32_t* err_word);
 /* Launch shape of the trace (the autotuner's knobs, kerrtrace_b200/autotune.py).  For the
  * persistent schedule: resident blocks of 128 threads per SM (3..6; the compiler caps registers
- * per thread accordingly; only the FP32 reference-semantics kernel has the 3/5/6 variants) and
- * the refill threshold.  For the plain schedule: the block shape (at most 1024 threads).
+ * per thread accordingly; only the FP32 reference-semantics kernel has the 3/5/6 variants).  For the plain schedule: the block shape (at most 1024 threads).
  * kt_trace(KT_SCHED_AUTO) runs tuning->schedule; the explicit schedules use the rest of the
  * tuning too, the pixel order included.  Default: wavefront, config block_dim, 4 blocks per
  * SM, refill 1, tile order.  Call it outside stream capture: the first long-first tuning of a
@@ -276,7 +276,7 @@ kt_status kt_context_get_tuning(const kt_context* ctx, kt_tuning* tuning);
  * for bit the first candidate's, and installs the fastest of those in the context
  * (kt_context_set_tuning); kt_trace(KT_SCHED_AUTO) then runs it.  candidates == NULL uses the
  * built-in list (plain block shapes, 128-thread plain blocks with more resident blocks per SM,
- * wavefront blocks per SM x refill thresholds, each in tile and long-rays-first order; at most
+ * wavefront blocks per SM, each in tile and long-rays-first order; at most
  * KT_TUNE_MAX_CANDIDATES, keep_frozen taken from the current tuning).  table (may be NULL)
  * receives one row per candidate, *n_entries their number.  Allocates scratch for one frame
  * and synchronises `stream`; call it at set-up, outside stream capture. */

@@ -2,8 +2,8 @@
 
 The tuner itself is C++ (kerrtrace_b200/csrc/kt_tune.cpp), so that any host of the C ABI can
 run it.  It times the trace of one view under each candidate launch shape (plain block shapes,
-128-thread plain blocks with more resident blocks per SM, persistent wavefront blocks per SM x
-refill thresholds, each in tile and long-rays-first order) with CUDA events, keeps only the
+128-thread plain blocks with more resident blocks per SM, persistent wavefront blocks per SM,
+each in tile and long-rays-first order) with CUDA events, keeps only the
 candidates whose image is bit for bit the first candidate's, and installs the fastest of those
 in the context; KT_SCHED_AUTO then runs it.
 """

@@ -7,7 +7,7 @@
 // The arithmetic of each formula is kept in the reference's order (same products, same
 // fused multiply-adds, same fast-math intrinsics) so that the FP32 path reproduces the
 // reference kernel's results; the scheduling around it (attempt-granular state machine,
-// persistent refill, retirement of NaN-frozen rays) is this project's.
+// persistent units, retirement of NaN-frozen rays) is this project's.
 //
 // Everything is templated on the integration type R (float for the reference arithmetic,
 // double for the FP64 path); the mixed path uses float RHS with a double state update.
@@ -29,6 +29,7 @@ template <> struct Ops<float> {
     static __device__ __forceinline__ float fdiv(float a, float b) { return __fdividef(a, b); }
     static __device__ __forceinline__ float sqrt_rn(float x) { return __fsqrt_rn(x); }
     static __device__ __forceinline__ float fma(float a, float b, float c) { return fmaf(a, b, c); }
+    static __device__ __forceinline__ float mul(float a, float b) { return __fmul_rn(a, b); }  // never contracted
     static __device__ __forceinline__ float powr(float a, float b) { return __powf(a, b); }
     static __device__ __forceinline__ float maxr(float a, float b) { return fmaxf(a, b); }
     static __device__ __forceinline__ float minr(float a, float b) { return fminf(a, b); }
@@ -44,6 +45,7 @@ template <> struct Ops<double> {
     static __device__ __forceinline__ double fdiv(double a, double b) { return a / b; }
     static __device__ __forceinline__ double sqrt_rn(double x) { return sqrt(x); }
     static __device__ __forceinline__ double fma(double a, double b, double c) { return ::fma(a, b, c); }
+    static __device__ __forceinline__ double mul(double a, double b) { return __dmul_rn(a, b); }
     static __device__ __forceinline__ double powr(double a, double b) { return pow(a, b); }
     static __device__ __forceinline__ double maxr(double a, double b) { return fmax(a, b); }
     static __device__ __forceinline__ double minr(double a, double b) { return fmin(a, b); }

@@ -20,8 +20,7 @@ struct PostParams {
 };
 
 // Tuning of the persistent tracer: resident blocks per SM (3..6 for the FP32 reference
-// kernel; the default otherwise) and the number of idle lanes a warp waits for before it
-// refills them (1..32).
+// kernel; the default otherwise).  refill_min is carried for its callers and has no effect.
 struct Tuning {
     int schedule = 1;
     int block_x = 0, block_y = 0;

@@ -7,9 +7,8 @@
 // Trace kernels (replace trace_kernel, cuda/kernel.cu:88-142):
 //   trace_plain_kernel      one thread per pixel on a 2D grid of block_dim tiles; each thread
 //                           runs its spp rays to completion through the attempt state machine.
-//   trace_wavefront_kernel  persistent: one block per resident slot, each lane owns a pixel and
-//                           pulls a new one from a device work counter (warp-aggregated atomics)
-//                           as soon as its rays are done, so long rays never idle a whole warp.
+//   trace_wavefront_kernel  persistent: one block per resident slot, each warp takes units of 32
+//                           rays (pixels x samples) from a device work counter.
 // Post kernels (replace bloom_horizontal / post_process, cuda/kernel.cu:144-251):
 //   bloom_h_kernel          horizontal normalised Gaussian, register-blocked over staged rows
 //   post_v_kernel           vertical Gaussian streamed from the bloom buffer + composite, ACES,
@@ -53,16 +52,18 @@ __device__ __forceinline__ void write_aux(float4* aux, size_t idx, const Tally& 
     if (aux) aux[idx] = make_float4(t.first_r, t.first_g, t.first_T, (float)t.hits);
 }
 
-// Runs one ray to completion (plain schedule).
-template <class R, int MODE, bool COUNT>
+// Runs one ray to completion and adds its colour to acc (A: float, or the ray's colour type).
+// later_sample: see ray_start.
+template <class R, int MODE, bool COUNT, class A>
 __device__ __forceinline__ void run_ray(int px, int py, int smp, const Scene& sc, const Camera& cam,
-                                        uint32_t* err, float acc[3], Tally& total, float4* aux) {
+                                        uint32_t* err, A acc[3], Tally& total, float4* aux,
+                                        bool later_sample = false) {
     float dir[3];
     pixel_ray<MODE>(px, py, smp, sc, cam, dir);
     RayRun<R> ry;
     Tally tl;
     tl.clear();
-    if (start(ry, cam, dir, sc)) {
+    if (start(ry, cam, dir, sc, later_sample)) {
         while (!advance<MODE, COUNT>(ry, sc, err, tl)) {
         }
     }
@@ -91,6 +92,38 @@ __device__ __forceinline__ void unit_to_pixel(unsigned u, int W, int H, int& px,
     const int wt = min(16, W - col0);
     py = row0 + (int)(rem2 / (unsigned)wt);
     px = col0 + (int)(rem2 % (unsigned)wt);
+}
+
+// Unit index -> pixel in 16x16 tiles (raster order), Morton order inside a tile: an aligned run of
+// 32, 16, 8, ... indices is a patch of 8x4, 4x4, 4x2, ... pixels.  The index space covers whole
+// tiles, so at the right and bottom border it names pixels outside the frame.
+__device__ __forceinline__ void tile_to_pixel(unsigned idx, int W, int& px, int& py) {
+    const unsigned tiles_x = ((unsigned)W + 15u) >> 4;
+    const unsigned tile = idx >> 8, m = idx & 255u;
+    const unsigned ty = tile / tiles_x, tx = tile - ty * tiles_x;
+    const unsigned x = (m & 1u) | (m >> 1 & 2u) | (m >> 2 & 4u) | (m >> 3 & 8u);
+    const unsigned y = (m >> 1 & 1u) | (m >> 2 & 2u) | (m >> 3 & 4u) | (m >> 4 & 8u);
+    px = (int)(tx * 16u + x);
+    py = (int)(ty * 16u + y);
+}
+// Units of 32 / S pixels that cover a frame: whole tiles, or exactly its pixels when they come
+// from a pixel-order buffer.
+__host__ __device__ __forceinline__ unsigned unit_count(int W, int H, int S, bool ordered) {
+    const unsigned P = 32u / (unsigned)S;
+    const unsigned n = ordered ? (unsigned)W * (unsigned)H
+                               : ((unsigned)(W + 15) >> 4) * ((unsigned)(H + 15) >> 4) * 256u;
+    return (n + P - 1u) / P;
+}
+// Lanes per pixel of the persistent tracer: the largest S <= min(spp, 32) that keeps 15 of 16
+// lanes busy over the pixel's samples (S lanes take spp samples in ceil(spp / S) rounds, and
+// 32 mod S lanes have no pixel).
+static int samples_in_parallel(int spp) {
+    int best = 1;
+    for (int S = 2; S <= 32 && S <= spp; ++S) {
+        const long long used = (long long)(32 / S) * spp, lanes = 32ll * ((spp + S - 1) / S);
+        if (16 * used >= 15 * lanes) best = S;
+    }
+    return best;
 }
 
 // ---- long-rays-first pixel order -----------------------------------------------------------
@@ -232,93 +265,75 @@ __global__ void __launch_bounds__(MAXT, MINB)
     if (COUNT) add_tally(ctr, (uint64_t)sc.spp, total);
 }
 
-// Persistent wavefront tracer.  A lane whose pixel is done takes a new one from the work
-// counter; lanes are refilled together once at least `refill_min` of the warp's lanes are idle
-// (or when the warp has nothing else to do), which trades idle lanes against how often the
-// divergent start-up code runs.
+// Persistent tracer.  A warp takes units of P = 32 / S pixels and gives each pixel S lanes, one per
+// sample (S = samples_in_parallel(spp); 1 at spp 1), so that the rays of a warp start together
+// and, with S > 1, come from a smaller patch of the frame.  Its first unit is its own index in
+// the grid, the others come from a device counter, so a frame of no more units than warps
+// needs neither the counter nor its reset.  The samples of a pixel are added in sample order
+// (shuffles over its lanes), as the plain kernel's loop adds them: the same bits.
+//
+// What bounds it: the FP32 (FP64) pipes, as the plain kernel; lanes idle only while the last rays
+// of their own unit finish.  An earlier form refilled single lanes from the counter as their
+// rays ended: each refill ran the start-up code (ray set-up, first tolerance, first right-hand
+// side) for one lane of 32, which cost more than the idle lanes it filled.  Against it (trace and
+// post, default tuning): 1920x1080 reference 3.58 -> 2.30 ms (trace), 960x540 FP64 6.69 -> 4.39,
+// 1024^2 mixed 2.62 -> 1.70, two frames of 2100x900 at 4 samples 15.9 -> 7.39; 96x64 at 2 samples
+// 0.272 -> 0.098, where a pixel's samples used to run one after the other on one lane; with
+// frozen rays kept to the end 183 -> 173.
 template <class R, int MODE, bool COUNT, int MINB>
 __global__ void __launch_bounds__(kWavefrontBlock, MINB)
     trace_wavefront_kernel(const __grid_constant__ Scene sc, const Camera cam, float4* __restrict__ hdr,
                            uint32_t* __restrict__ err, unsigned* __restrict__ queue,
-                           unsigned long long* __restrict__ ctr, float4* __restrict__ aux,
-                           int refill_min, const unsigned* __restrict__ order) {
+                           unsigned long long* __restrict__ ctr, float4* __restrict__ aux, int S,
+                           const unsigned* __restrict__ order) {
     const int lane = threadIdx.x & 31;
-    const unsigned lane_lt = (1u << lane) - 1u;
-    const unsigned n_units = (unsigned)sc.width * (unsigned)sc.height;
+    const int slot = lane / S, sub = lane - slot * S;
+    const unsigned P = 32u / (unsigned)S;
+    const unsigned n_px = (unsigned)sc.width * (unsigned)sc.height;
+    const unsigned units = unit_count(sc.width, sc.height, S, order != nullptr);
     const unsigned n_hot = order ? order[0] : 0u;
-    RayRun<R> ry;
-    int px = 0, py = 0, smp = 0;
-    float acc[3] = {0.0f, 0.0f, 0.0f};
-    bool active = false;
-    bool open = true;
-    Tally tl, total;
-    tl.clear();
+    const unsigned n_warps = gridDim.x * (kWavefrontBlock / 32);
+    Tally total;
     total.clear();
     uint64_t rays = 0;
 
-    while (true) {
-        if (open) {
-            const unsigned need = __ballot_sync(kFull, !active);
-            const int idle = __popc(need);
-            if (idle >= refill_min || (idle > 0 && idle == 32)) {
-                const int leader = __ffs(need) - 1;
-                const unsigned cnt = (unsigned)idle;
-                unsigned base = 0;
-                if (lane == leader) base = atomicAdd(queue, cnt);
-                base = __shfl_sync(kFull, base, leader);
-                if (base + cnt >= n_units) open = false;
-                if (!active) {
-                    const unsigned u = base + (unsigned)__popc(need & lane_lt);
-                    if (u < n_units) {
-                        if (order)
-                            ordered_pixel(u, n_units, order, n_hot, sc.width, px, py);
-                        else
-                            unit_to_pixel(u, sc.width, sc.height, px, py);
-                        acc[0] = acc[1] = acc[2] = 0.0f;
-                        // first sample with work; samples whose loop would not run add zero
-                        for (smp = 0; smp < sc.spp; ++smp) {
-                            float dir[3];
-                            pixel_ray<MODE>(px, py, smp, sc, cam, dir);
-                            if (COUNT) tl.clear();
-                            if (start(ry, cam, dir, sc)) break;
-                        }
-                        if (smp < sc.spp) {
-                            active = true;
-                        } else {
-                            const float fs = sc.final_scale;
-                            hdr[py * sc.width + px] =
-                                make_float4(acc[0] * fs, acc[1] * fs, acc[2] * fs, 1.0f);
-                            if (COUNT) rays += (uint64_t)sc.spp;
-                        }
-                    }
+    for (unsigned u = blockIdx.x * (kWavefrontBlock / 32) + (threadIdx.x >> 5); u < units;) {
+        const unsigned idx = u * P + (unsigned)slot;
+        int px = 0, py = 0;
+        bool valid = (unsigned)slot < P;
+        if (order) {
+            valid = valid && idx < n_px;
+            if (valid) ordered_pixel(idx, n_px, order, n_hot, sc.width, px, py);
+        } else {
+            tile_to_pixel(idx, sc.width, px, py);
+            valid = valid && px < sc.width && py < sc.height;
+        }
+        float acc[3] = {0.0f, 0.0f, 0.0f};
+        for (int s0 = 0; s0 < sc.spp; s0 += S) {
+            decltype(RayRun<R>::tau) col[3] = {0, 0, 0};
+            if (valid && s0 + sub < sc.spp) {
+                run_ray<R, MODE, COUNT>(px, py, s0 + sub, sc, cam, err, col, total, aux, s0 + sub > 0);
+                if (COUNT) ++rays;
+            }
+            __syncwarp();
+            if (S == 1) {
+#pragma unroll
+                for (int c = 0; c < 3; ++c) acc[c] += col[c];
+            } else {
+                const int last = min(S, sc.spp - s0);
+                for (int i = 0; i < last; ++i) {
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) acc[c] += __shfl_sync(kFull, col[c], min(slot * S + i, 31));
                 }
             }
         }
-        if (!__any_sync(kFull, active)) {
-            if (!open) break;
-            continue;
+        if (valid && sub == 0) {
+            const float fs = sc.final_scale;
+            hdr[py * sc.width + px] = make_float4(acc[0] * fs, acc[1] * fs, acc[2] * fs, 1.0f);
         }
-        if (active && advance<MODE, COUNT>(ry, sc, err, tl)) {
-            acc[0] += ry.col[0];
-            acc[1] += ry.col[1];
-            acc[2] += ry.col[2];
-            if (COUNT) {
-                tally_ray(total, tl);
-                if (smp == 0) write_aux(aux, (size_t)py * sc.width + px, tl);
-            }
-            for (++smp; smp < sc.spp; ++smp) {
-                float dir[3];
-                pixel_ray<MODE>(px, py, smp, sc, cam, dir);
-                if (COUNT) tl.clear();
-                if (start(ry, cam, dir, sc)) break;
-            }
-            if (smp >= sc.spp) {
-                const float fs = sc.final_scale;
-                hdr[py * sc.width + px] = make_float4(acc[0] * fs, acc[1] * fs, acc[2] * fs, 1.0f);
-                if (COUNT) rays += (uint64_t)sc.spp;
-                active = false;
-            }
-        }
+        if (units <= n_warps) break;
+        if (lane == 0) u = n_warps + atomicAdd(queue, 1u);
+        u = __shfl_sync(kFull, u, 0);
     }
     if (COUNT) add_tally(ctr, rays, total);
 }
@@ -367,21 +382,24 @@ static cudaError_t launch_plain(const Scene& sc, const Camera& cam, float4* hdr,
 
 template <class R, int MODE, bool COUNT, int MINB>
 static cudaError_t launch_wave_minb(const Scene& sc, const Camera& cam, float4* hdr, uint32_t* err,
-                                    unsigned* queue, unsigned long long* ctr, float4* aux, int refill,
-                                    const unsigned* order, cudaStream_t st) {
-    int dev = 0, sms = 0, per_sm = 0;
+                                    unsigned* queue, unsigned long long* ctr, float4* aux, const unsigned* order,
+                                    cudaStream_t st) {
+    int dev = 0, sms = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
     e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess) return e;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, trace_wavefront_kernel<R, MODE, COUNT, MINB>,
-                                                      kWavefrontBlock, 0);
-    if (e != cudaSuccess) return e;
-    if (per_sm < 1) per_sm = 1;
-    e = cudaMemsetAsync(queue, 0, sizeof(unsigned), st);
-    if (e != cudaSuccess) return e;
+    constexpr unsigned kWarps = kWavefrontBlock / 32;
+    const int S = samples_in_parallel(sc.spp);
+    const unsigned units = unit_count(sc.width, sc.height, S, order != nullptr);
+    const unsigned blocks = (units + kWarps - 1) / kWarps, resident = (unsigned)(sms * MINB);
+    const unsigned grid = blocks < resident ? blocks : resident;
+    if (units > grid * kWarps) {
+        e = cudaMemsetAsync(queue, 0, sizeof(unsigned), st);
+        if (e != cudaSuccess) return e;
+    }
     trace_wavefront_kernel<R, MODE, COUNT, MINB>
-        <<<sms * per_sm, kWavefrontBlock, 0, st>>>(sc, cam, hdr, err, queue, ctr, aux, refill, order);
+        <<<grid, kWavefrontBlock, 0, st>>>(sc, cam, hdr, err, queue, ctr, aux, S, order);
     return cudaGetLastError();
 }
 
@@ -389,16 +407,15 @@ template <class R, int MODE, bool COUNT>
 static cudaError_t launch_wave(const Scene& sc, const Camera& cam, float4* hdr, uint32_t* err,
                                unsigned* queue, unsigned long long* ctr, float4* aux, const Tuning& tn,
                                const unsigned* order, cudaStream_t st) {
-    const int refill = tn.refill_min < 1 ? 1 : (tn.refill_min > 32 ? 32 : tn.refill_min);
     if constexpr (std::is_same<R, float>::value && MODE == 0 && !COUNT) {
         switch (tn.blocks_per_sm) {
-            case 3: return launch_wave_minb<R, MODE, COUNT, 3>(sc, cam, hdr, err, queue, ctr, aux, refill, order, st);
-            case 5: return launch_wave_minb<R, MODE, COUNT, 5>(sc, cam, hdr, err, queue, ctr, aux, refill, order, st);
-            case 6: return launch_wave_minb<R, MODE, COUNT, 6>(sc, cam, hdr, err, queue, ctr, aux, refill, order, st);
+            case 3: return launch_wave_minb<R, MODE, COUNT, 3>(sc, cam, hdr, err, queue, ctr, aux, order, st);
+            case 5: return launch_wave_minb<R, MODE, COUNT, 5>(sc, cam, hdr, err, queue, ctr, aux, order, st);
+            case 6: return launch_wave_minb<R, MODE, COUNT, 6>(sc, cam, hdr, err, queue, ctr, aux, order, st);
             default: break;
         }
     }
-    return launch_wave_minb<R, MODE, COUNT, WaveDefaults<R>::minb>(sc, cam, hdr, err, queue, ctr, aux, refill, order, st);
+    return launch_wave_minb<R, MODE, COUNT, WaveDefaults<R>::minb>(sc, cam, hdr, err, queue, ctr, aux, order, st);
 }
 
 template <class R, int MODE>

@@ -5,8 +5,7 @@
 // attempt granularity: ray_advance() performs exactly one attempt and, when the attempt ends
 // the step (accepted, or max_attempts reached), commits it and runs the horizon / disk-plane /
 // escape tests.  A warp whose lanes hold rays at different attempt counts therefore keeps all
-// lanes busy on the expensive part (six RHS evaluations), and a lane whose ray has ended can be
-// refilled with a new ray without waiting for its neighbours.
+// lanes busy on the expensive part (six RHS evaluations).
 //
 // MODE: 0 reference semantics (LUTs through texture objects), 1 stated physics, 2 reference
 // semantics with the LUTs read from plain device arrays through a model of the texture unit.
@@ -97,9 +96,15 @@ __device__ __forceinline__ void pixel_ray(int px, int py, int sample, const Scen
 // Null initialisation (cuda/kerr_trace.cuh:14-47): p_t from the null condition with the
 // "-sqrt" root, covariant spatial momentum p = n + 2 Hk l (k_t + l.n).  Returns false when
 // the step loop would not run at all.
+//
+// N_z = r z + a x is a sum of two products, so it has two fused forms, which differ in the last
+// place for some camera positions.  The reference kernel's, and the plain schedule's, is
+// fma(a, x, r z).  The persistent schedules start the second and later samples of a pixel with
+// fma(r, z, a x) (later_sample): an ulp in l_z, which moves a sky line by a pixel here and there.
+// Both are written out so that each schedule keeps its own image bits.
 template <class R>
 __device__ __forceinline__ bool ray_start(RayRun<R>& ry, const Camera& cam, const float dir[3],
-                                          const Scene& sc) {
+                                          const Scene& sc, bool later_sample = false) {
     using O = Ops<R>;
     const R a = sc_a<R>(sc), aa = sc_aa<R>(sc), M = sc_M<R>(sc);
     const R dx = (R)dir[0], dy = (R)dir[1], dz = (R)dir[2];
@@ -113,9 +118,10 @@ __device__ __forceinline__ bool ray_start(RayRun<R>& ry, const Camera& cam, cons
     const R r = O::sqrt_rn(r2);
     const R den = r2 + aa;
     const R inv_den = O::fdiv(R(1), den);
-    const R lx = (r * x - a * z) * inv_den;
+    const R lx = O::mul(O::fma(r, x, -O::mul(a, z)), inv_den);
     const R ly = O::fdiv(y, r);
-    const R lz = (r * z + a * x) * inv_den;
+    const R Nz = later_sample ? O::fma(r, z, O::mul(a, x)) : O::fma(a, x, O::mul(r, z));
+    const R lz = O::mul(Nz, inv_den);
     const R denH = O::fma(r2, r2, aa * y * y);
     const R Hk = M * r2 * r * O::fdiv(R(1), denH);
     const R ln = O::fma(lx, nx, O::fma(ly, ny, lz * nz));
@@ -510,9 +516,9 @@ __device__ __forceinline__ void null_renormalise(double* s, double pt, const Sce
 // The start is the FP32 start (the camera and direction are FP32 data; it runs once per ray in
 // the refill path, where FP64 square roots and divisions would cost as much as the ray's steps).
 __device__ __forceinline__ bool ray_start_mixed(RayRun<Mixed>& ry, const Camera& cam, const float dir[3],
-                                                const Scene& sc) {
+                                                const Scene& sc, bool later_sample) {
     RayRun<float> d;
-    const bool run = ray_start<float>(d, cam, dir, sc);
+    const bool run = ray_start<float>(d, cam, dir, sc, later_sample);
 #pragma unroll
     for (int c = 0; c < 6; ++c) {
         ry.s[c] = d.s[c];
@@ -756,11 +762,13 @@ __device__ __forceinline__ bool ray_advance_mixed(RayRun<Mixed>& ry, const Scene
 
 // Uniform entry points used by the kernels for every arithmetic type.
 template <class R>
-__device__ __forceinline__ bool start(RayRun<R>& ry, const Camera& cam, const float dir[3], const Scene& sc) {
-    return ray_start<R>(ry, cam, dir, sc);
+__device__ __forceinline__ bool start(RayRun<R>& ry, const Camera& cam, const float dir[3], const Scene& sc,
+                                      bool later_sample = false) {
+    return ray_start<R>(ry, cam, dir, sc, later_sample);
 }
-__device__ __forceinline__ bool start(RayRun<Mixed>& ry, const Camera& cam, const float dir[3], const Scene& sc) {
-    return ray_start_mixed(ry, cam, dir, sc);
+__device__ __forceinline__ bool start(RayRun<Mixed>& ry, const Camera& cam, const float dir[3], const Scene& sc,
+                                      bool later_sample = false) {
+    return ray_start_mixed(ry, cam, dir, sc, later_sample);
 }
 template <int MODE, bool COUNT, class R>
 __device__ __forceinline__ bool advance(RayRun<R>& ry, const Scene& sc, uint32_t* err, Tally& tl) {

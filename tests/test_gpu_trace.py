@@ -252,3 +252,16 @@ def test_keep_frozen_rays_is_bit_identical(cuda, schedule):
     # every frozen ray now runs out its step budget
     assert sb.steps - sa.steps >= sb.frozen_rays * cfg.max_steps // 2, (sa.steps, sb.steps, sb.frozen_rays)
     ctx.close()
+
+
+@pytest.mark.parametrize("size,spp", [((1, 1), 1), ((17, 33), 1), ((257, 15), 1), ((96, 64), 3), ((31, 7), 8),
+                                      ((48, 20), 17), ((9, 5), 33)])
+def test_persistent_units_match_plain(cuda, size, spp):
+    """The persistent schedule's units (whole 16x16 tiles, several lanes per pixel at spp > 1, more
+    samples than lanes) give the plain schedule's image on the t1 view, bit for bit."""
+    cfg, cam = workloads.scene("t1")
+    cfg = workloads.scaled(cfg, *size)
+    cfg.spp = spp
+    a, _, _, ctx = run_ours(cuda, cfg, cam, kt.SCHED_PLAIN)
+    b, _, _, _ = run_ours(cuda, cfg, cam, kt.SCHED_WAVEFRONT, ctx=ctx)
+    assert np.array_equal(a.view(np.uint32), b.view(np.uint32))
