@@ -303,7 +303,6 @@ __device__ __forceinline__ bool ray_begin(int px, int py, const Scene& sc, const
         ry.tau = 1.0;
         ry.step = 0;
         ry.attempt = 0;
-        ry.have_k1 = false;
         return 0 < sc.max_steps && 1.0f > sc.cutoff_gt;
     }
 }
@@ -429,6 +428,7 @@ __global__ void __launch_bounds__(128, 4) diff_forward_kernel(const Scene sc, co
             int cur = -1, in_seg = 0;
             bool rec_ok = true;
             DiffSeg<R>* sg = nullptr;
+            prepare<1, true>(ry, sc, tl);
             while (true) {
                 if (ry.attempt == 0 && in_seg == 0 && rec_ok) {  // a step starts a new segment
                     const unsigned idx = atomicAdd(rec.seg_count, 1u);
@@ -452,7 +452,7 @@ __global__ void __launch_bounds__(128, 4) diff_forward_kernel(const Scene sc, co
                 }
                 const R h_used = ry.h;
                 const uint32_t hits0 = tl.hits;
-                const bool done = advance<1, true>(ry, sc, err, tl);
+                const bool done = advance<1, true>(ry, sc, err, tl) != kRayGoing;
                 if (ry.attempt != 0) continue;  // rejected attempt: the step is retried
                 if (Ops<R>::isnanr(ry.s[1])) {  // frozen: this step is not part of the record
                     out.term = kTermFrozen;
@@ -490,11 +490,12 @@ __global__ void __launch_bounds__(128, 4) diff_forward_kernel(const Scene sc, co
         if (started != (rr.term != kTermNotStarted)) flip = 1;
         if (started && rr.term != kTermNotStarted && rr.term != kTermOverflow) {
             bool done = false;
+            prepare<1, true>(ry, sc, tl);
             for (int si = rr.first_seg; si >= 0 && !done; si = seg_at<RR>(rec, si)->next) {
                 const DiffSeg<RR>* sg = seg_at<RR>(rec, si);
                 for (int j = 0; j < sg->n && !done; ++j) {
                     ry.h = (R)sg->h[j];
-                    done = advance<1, true>(ry, sc, err, tl);  // one attempt: always a commit
+                    done = advance<1, true>(ry, sc, err, tl) != kRayGoing;  // one attempt: always a commit
                     ++n_done;
                 }
             }

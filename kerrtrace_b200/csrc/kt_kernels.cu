@@ -52,21 +52,23 @@ __device__ __forceinline__ void write_aux(float4* aux, size_t idx, const Tally& 
     if (aux) aux[idx] = make_float4(t.first_r, t.first_g, t.first_T, (float)t.hits);
 }
 
-// Runs one ray to completion and adds its colour to acc (A: float, or the ray's colour type).
-// later_sample: see ray_start.
-template <class R, int MODE, bool COUNT, class A>
-__device__ __forceinline__ void run_ray(int px, int py, int smp, const Scene& sc, const Camera& cam,
-                                        uint32_t* err, A acc[3], Tally& total, float4* aux,
+// Runs one ray per lane to completion and adds its colour to acc (A: float, or the ray's colour
+// type).  active: the lane has a ray; later_sample: see ray_start; TOGETHER: see run_rays.
+template <class R, int MODE, bool COUNT, bool TOGETHER, class A>
+__device__ __forceinline__ void run_ray(bool active, int px, int py, int smp, const Scene& sc,
+                                        const Camera& cam, uint32_t* err, A acc[3], Tally& total, float4* aux,
                                         bool later_sample = false) {
-    float dir[3];
-    pixel_ray<MODE>(px, py, smp, sc, cam, dir);
     RayRun<R> ry;
     Tally tl;
     tl.clear();
-    if (start(ry, cam, dir, sc, later_sample)) {
-        while (!advance<MODE, COUNT>(ry, sc, err, tl)) {
-        }
+    bool run = false;
+    if (active) {
+        float dir[3];
+        pixel_ray<MODE>(px, py, smp, sc, cam, dir);
+        run = start(ry, cam, dir, sc, later_sample);
     }
+    run_rays<MODE, COUNT, TOGETHER>(run, ry, sc, err, tl);
+    if (!active) return;
     acc[0] += ry.col[0];
     acc[1] += ry.col[1];
     acc[2] += ry.col[2];
@@ -258,7 +260,8 @@ __global__ void __launch_bounds__(MAXT, MINB)
     Tally total;
     total.clear();
     const int s_end = sc.sample_first + sc.spp;
-    for (int smp = sc.sample_first; smp < s_end; ++smp) run_ray<R, MODE, COUNT>(px, py, smp, sc, cam, err, acc, total, aux);
+    for (int smp = sc.sample_first; smp < s_end; ++smp)
+        run_ray<R, MODE, COUNT, false>(true, px, py, smp, sc, cam, err, acc, total, aux);
     if (sc.accum) sc.accum[pix] = make_float4(acc[0], acc[1], acc[2], (float)s_end);
     const float fs = sc.final_scale;
     hdr[pix] = make_float4(acc[0] * fs, acc[1] * fs, acc[2] * fs, 1.0f);
@@ -280,7 +283,7 @@ __global__ void __launch_bounds__(MAXT, MINB)
 // 1024^2 mixed 2.62 -> 1.70, two frames of 2100x900 at 4 samples 15.9 -> 7.39; 96x64 at 2 samples
 // 0.272 -> 0.098, where a pixel's samples used to run one after the other on one lane; with
 // frozen rays kept to the end 183 -> 173.
-template <class R, int MODE, bool COUNT, int MINB>
+template <class R, int MODE, bool COUNT, int MINB, bool TOGETHER>
 __global__ void __launch_bounds__(kWavefrontBlock, MINB)
     trace_wavefront_kernel(const __grid_constant__ Scene sc, const Camera cam, float4* __restrict__ hdr,
                            uint32_t* __restrict__ err, unsigned* __restrict__ queue,
@@ -311,11 +314,9 @@ __global__ void __launch_bounds__(kWavefrontBlock, MINB)
         float acc[3] = {0.0f, 0.0f, 0.0f};
         for (int s0 = 0; s0 < sc.spp; s0 += S) {
             decltype(RayRun<R>::tau) col[3] = {0, 0, 0};
-            if (valid && s0 + sub < sc.spp) {
-                run_ray<R, MODE, COUNT>(px, py, s0 + sub, sc, cam, err, col, total, aux, s0 + sub > 0);
-                if (COUNT) ++rays;
-            }
-            __syncwarp();
+            const bool has_sample = valid && s0 + sub < sc.spp;
+            run_ray<R, MODE, COUNT, TOGETHER>(has_sample, px, py, s0 + sub, sc, cam, err, col, total, aux, s0 + sub > 0);
+            if (COUNT && has_sample) ++rays;
             if (S == 1) {
 #pragma unroll
                 for (int c = 0; c < 3; ++c) acc[c] += col[c];
@@ -398,7 +399,18 @@ static cudaError_t launch_wave_minb(const Scene& sc, const Camera& cam, float4* 
         e = cudaMemsetAsync(queue, 0, sizeof(unsigned), st);
         if (e != cudaSuccess) return e;
     }
-    trace_wavefront_kernel<R, MODE, COUNT, MINB>
+    // At most one unit per resident warp: the launch lasts as long as its longest rays, and the warp
+    // that keeps its lanes in step issues fewer instructions for them (96x64 x 2 samples 78.3 -> 72.2
+    // us, 256x256 at tolerance 1e-8 23.9 -> 23.3 ms).  With more units the vote and the register
+    // moves around it cost more than they save (1920x1080 2.21 -> 2.37 ms).
+    if constexpr (!COUNT && MINB == WaveDefaults<R>::minb) {
+        if (units <= resident * kWarps) {
+            trace_wavefront_kernel<R, MODE, COUNT, MINB, true>
+                <<<grid, kWavefrontBlock, 0, st>>>(sc, cam, hdr, err, queue, ctr, aux, S, order);
+            return cudaGetLastError();
+        }
+    }
+    trace_wavefront_kernel<R, MODE, COUNT, MINB, false>
         <<<grid, kWavefrontBlock, 0, st>>>(sc, cam, hdr, err, queue, ctr, aux, S, order);
     return cudaGetLastError();
 }
@@ -463,7 +475,8 @@ __global__ void __launch_bounds__(MAXT, MAXT == 256 ? PlainMinBlocks<R>::v : 1)
     float acc[3] = {0.0f, 0.0f, 0.0f};
     Tally total;
     total.clear();
-    for (int smp = 0; smp < sc.spp; ++smp) run_ray<R, MODE, false>(px, py, smp, sc, jb.cam, jb.err, acc, total, nullptr);
+    for (int smp = 0; smp < sc.spp; ++smp)
+        run_ray<R, MODE, false, false>(true, px, py, smp, sc, jb.cam, jb.err, acc, total, nullptr);
     const float fs = sc.final_scale;
     jb.hdr[py * sc.width + px] = make_float4(acc[0] * fs, acc[1] * fs, acc[2] * fs, 1.0f);
 }
@@ -509,14 +522,15 @@ __global__ void __launch_bounds__(kWavefrontBlock, MINB)
         const BatchJob& jb = bt.job[lo];
         const Scene& sc = jb.sc;
         const unsigned pix = (u - jb.unit_begin) * 32u + (unsigned)lane;
-        if (pix < (unsigned)sc.width * (unsigned)sc.height) {
-            int px, py;
-            unit_to_pixel(pix, sc.width, sc.height, px, py);
-            float acc[3] = {0.0f, 0.0f, 0.0f};
-            Tally total;
-            total.clear();
-            for (int smp = 0; smp < sc.spp; ++smp)
-                run_ray<R, MODE, false>(px, py, smp, sc, jb.cam, jb.err, acc, total, nullptr);
+        const bool valid = pix < (unsigned)sc.width * (unsigned)sc.height;
+        int px = 0, py = 0;
+        if (valid) unit_to_pixel(pix, sc.width, sc.height, px, py);
+        float acc[3] = {0.0f, 0.0f, 0.0f};
+        Tally total;
+        total.clear();
+        for (int smp = 0; smp < sc.spp; ++smp)
+            run_ray<R, MODE, false, false>(valid, px, py, smp, sc, jb.cam, jb.err, acc, total, nullptr);
+        if (valid) {
             const float fs = sc.final_scale;
             jb.hdr[py * sc.width + px] = make_float4(acc[0] * fs, acc[1] * fs, acc[2] * fs, 1.0f);
         }

@@ -103,6 +103,7 @@ __global__ void __launch_bounds__(kNoallocBlock, 4)
                             if (ray_start<float>(ry, cam, dir, sc)) break;
                         }
                         if (smp < sc.spp) {
+                            ray_prepare<float, MODE, false>(ry, sc, tl);
                             active = true;
                         } else {
                             const float fs = sc.final_scale;
@@ -120,7 +121,8 @@ __global__ void __launch_bounds__(kNoallocBlock, 4)
             if (!open) break;
             continue;
         }
-        if (active && ray_advance<float, MODE, false>(ry, sc, err + 2 * lview, tl)) {
+        const int state = active ? ray_advance<float, MODE, false, false>(ry, sc, err + 2 * lview, tl, kRayGoing) : kRayGoing;
+        if (state != kRayGoing) {
             acc[0] += ry.col[0];
             acc[1] += ry.col[1];
             acc[2] += ry.col[2];
@@ -130,6 +132,7 @@ __global__ void __launch_bounds__(kNoallocBlock, 4)
                 pixel_ray<MODE>(px, py, smp, sc, cam, dir);
                 if (ray_start<float>(ry, cam, dir, sc)) break;
             }
+            if (smp < sc.spp) ray_prepare<float, MODE, false>(ry, sc, tl);
             if (smp >= sc.spp) {
                 const float fs = sc.final_scale;
                 hdr[(size_t)lview * n_units + (size_t)py * sc.width + px] =

@@ -50,16 +50,21 @@ template <> __device__ __forceinline__ bool tau_alive<double>(double tau, const 
 template <class R>
 struct RayRun {
     R s[6];      // x, y, z, p_x, p_y, p_z
-    R k1[6];     // RHS at s (valid when have_k1)
+    R k1[6];     // RHS at s
     R pt, kt, h, tol;
     R col[3];    // colour and transmittance: float on the float paths, double on the FP64 path
     R tau;
     int step;    // committed steps (the reference's loop index i)
     int attempt; // attempts spent on the current step
-    bool have_k1;
 };
 
-// Work counters of one ray (only maintained by the counting kernels).
+// What an attempt left the ray in.
+enum RayState : int {
+    kRayGoing = 0,
+    kRayDone = 1,     // the colour is final
+    kRayEscaped = 2,  // ended beyond the escape radius: ray_finish adds the sky
+};
+
 // Work counters of one ray, and the first shaded disk hit (only maintained by the counting
 // kernels).
 struct Tally {
@@ -146,7 +151,6 @@ __device__ __forceinline__ bool ray_start(RayRun<R>& ry, const Camera& cam, cons
     ry.tau = 1.0f;
     ry.step = 0;
     ry.attempt = 0;
-    ry.have_k1 = false;
     return 0 < sc.max_steps && 1.0f > sc.cutoff_gt;
 }
 
@@ -332,22 +336,47 @@ __device__ __forceinline__ void shade_crossing(RayRun<R>& ry, const R* prev, con
     shade_hit<R, MODE>(hit, ry.pt, ry.kt, ry.col, ry.tau, sc, err, tl);
 }
 
-// One DP5(4) attempt; on the last attempt of a step, the commit and the per-step tests.
-// Returns true when the ray has finished (its colour is final).
+// Tolerance and right-hand side of a ray's first step (later steps get theirs from the commit of
+// the step before), ahead of the attempt loop: inside it, behind a test, they cost the loop registers
+// and instructions (trace of 1920x1080 2.255 -> 2.188 ms in the tuned shape, 1024^2 mixed 1.81 ->
+// 1.14 in the persistent one).  The start state is hidden from the optimiser: it knows the position for the
+// camera's, and would share parts of the right-hand side with the ray's start, fused differently
+// from the copy in the loop.
+__device__ __forceinline__ void opaque(float& v) { asm volatile("" : "+f"(v)); }
+__device__ __forceinline__ void opaque(double& v) { asm volatile("" : "+d"(v)); }
 template <class R, int MODE, bool COUNT>
-__device__ __forceinline__ bool ray_advance(RayRun<R>& ry, const Scene& sc, uint32_t* err,
-                                            Tally& tl) {
+__device__ __forceinline__ void ray_prepare(RayRun<R>& ry, const Scene& sc, Tally& tl) {
+#pragma unroll
+    for (int c = 0; c < 6; ++c) opaque(ry.s[c]);
+    ry.tol = step_tolerance<R, MODE>(ry.s, sc);
+    hamilton_rhs<R, MODE == 1>(ry.s, ry.pt, sc_a<R>(sc), sc_aa<R>(sc), sc_M<R>(sc), ry.k1);
+    if (COUNT) tl.rhs++;
+}
+
+// Sky in the direction of an escaped ray.
+template <class R, int MODE, bool COUNT>
+__device__ __forceinline__ void ray_sky(RayRun<R>& ry, const Scene& sc, Tally& tl) {
+    using O = Ops<R>;
+    R ke[6];
+    hamilton_rhs<R, MODE == 1>(ry.s, ry.pt, sc_a<R>(sc), sc_aa<R>(sc), sc_M<R>(sc), ke);
+    if (COUNT) tl.rhs++;
+    const R inv = O::rsq(ke[0] * ke[0] + ke[1] * ke[1] + ke[2] * ke[2]);
+    const R sky = sky_value<R>(ke[0] * inv, ke[1] * inv, ke[2] * inv, ry.tau, sc);
+    ry.col[0] += sky;
+    ry.col[1] += sky;
+    ry.col[2] += sky;
+}
+
+// One DP5(4) attempt; on the last attempt of a step, the commit and the per-step tests.
+// TOGETHER (run_rays): the ray may already have ended (its attempt is computed and dropped), and
+// the sky of an escaped ray is left to the caller.
+template <class R, int MODE, bool COUNT, bool TOGETHER>
+__device__ __forceinline__ int ray_advance(RayRun<R>& ry, const Scene& sc, uint32_t* err,
+                                           Tally& tl, int state) {
     constexpr bool EXACT = MODE == 1;
     using O = Ops<R>;
     using C = DP<R>;
     const R a = sc_a<R>(sc), aa = sc_aa<R>(sc), M = sc_M<R>(sc);
-    // the first step's tolerance; later steps get theirs from the commit of the step before
-    if (ry.attempt == 0 && ry.step == 0) ry.tol = step_tolerance<R, MODE>(ry.s, sc);
-    if (!ry.have_k1) {
-        hamilton_rhs<R, EXACT>(ry.s, ry.pt, a, aa, M, ry.k1);
-        ry.have_k1 = true;
-        if (COUNT) tl.rhs++;
-    }
     const R h = ry.h;
     const R* s = ry.s;
     const R* k1 = ry.k1;
@@ -388,11 +417,13 @@ __device__ __forceinline__ bool ray_advance(RayRun<R>& ry, const Scene& sc, uint
     const bool ok = errv <= R(1);
     ry.h = h * lit<R>(0.9f, 0.9) * O::powr(errv, lit<R>(-0.2f, -0.2));
     ry.attempt++;
-    if (COUNT) {
+    const bool going = !TOGETHER || state == kRayGoing;
+    if (COUNT && going) {
         tl.attempts++;
         tl.rhs += 6;
     }
-    if (!ok && ry.attempt < sc.max_attempts) return false;  // retry; k1 stays valid at s
+    if (TOGETHER && !going) return state;
+    if (!ok && ry.attempt < sc.max_attempts) return kRayGoing;  // retry; k1 stays valid at s
 
     // commit (also when every attempt was rejected: cuda/kerr_trace.cuh:123-134)
     R prev[6];
@@ -405,34 +436,37 @@ __device__ __forceinline__ bool ray_advance(RayRun<R>& ry, const Scene& sc, uint
     if (COUNT) tl.steps++;
     if (O::isnanr(ry.s[1])) {  // frozen: no later comparison can succeed (see file comment)
         if (COUNT) tl.frozen = 1;
-        if (!sc.keep_frozen) return true;
+        if (!sc.keep_frozen) return kRayDone;
     }
     const R r_now = ks_radius<R>(ry.s[0], ry.s[1], ry.s[2], aa);
-    if (inside_horizon<R>(r_now, sc)) return true;
+    if (inside_horizon<R>(r_now, sc)) return kRayDone;
     if ((prev[1] < R(0) && ry.s[1] >= R(0)) || (prev[1] > R(0) && ry.s[1] <= R(0)))
         shade_crossing<R, MODE>(ry, prev, ry.k1, k3, k4, k5, k6, k7, h, sc, err, COUNT ? &tl : nullptr);
-    if (ok) {
 #pragma unroll
-        for (int c = 0; c < 6; ++c) ry.k1[c] = k7[c];
-        ry.have_k1 = true;
-    } else {
-        ry.have_k1 = false;
-    }
+    for (int c = 0; c < 6; ++c) ry.k1[c] = k7[c];
     if (beyond_escape<R>(r_now, sc)) {
-        R ke[6];
-        hamilton_rhs<R, EXACT>(ry.s, ry.pt, a, aa, M, ke);
-        if (COUNT) tl.rhs++;
-        const R inv = O::rsq(ke[0] * ke[0] + ke[1] * ke[1] + ke[2] * ke[2]);
-        const R sky = sky_value<R>(ke[0] * inv, ke[1] * inv, ke[2] * inv, ry.tau, sc);
-        ry.col[0] += sky;
-        ry.col[1] += sky;
-        ry.col[2] += sky;
-        return true;
+        if (TOGETHER) return kRayEscaped;
+        if constexpr (MODE == 1) {
+            ray_sky<R, MODE, COUNT>(ry, sc, tl);
+        } else {  // ray_sky spelled out: as a call the 80-register kernel spills 40 bytes (2.29 -> 2.19 ms at 1080p)
+            R ke[6];
+            hamilton_rhs<R, EXACT>(ry.s, ry.pt, a, aa, M, ke);
+            if (COUNT) tl.rhs++;
+            const R inv = O::rsq(ke[0] * ke[0] + ke[1] * ke[1] + ke[2] * ke[2]);
+            const R sky = sky_value<R>(ke[0] * inv, ke[1] * inv, ke[2] * inv, ry.tau, sc);
+            ry.col[0] += sky;
+            ry.col[1] += sky;
+            ry.col[2] += sky;
+        }
+        return kRayDone;
     }
+    // after a forced commit the reference evaluates the right-hand side again
+    if (!ok) hamilton_rhs<R, EXACT>(ry.s, ry.pt, a, aa, M, ry.k1);
     ry.step++;
-    const bool done = !(ry.step < sc.max_steps && tau_alive<R>(ry.tau, sc));
-    if (!done) ry.tol = step_tolerance_at<R, MODE>(r_now, ry.s, sc);
-    return done;
+    if (!(ry.step < sc.max_steps && tau_alive<R>(ry.tau, sc))) return kRayDone;
+    ry.tol = step_tolerance_at<R, MODE>(r_now, ry.s, sc);
+    if (COUNT && !ok) tl.rhs++;
+    return kRayGoing;
 }
 
 // =========================================================================================
@@ -462,7 +496,7 @@ struct RayRun<Mixed> {
     float col[3];
     float tau;
     int step, attempt;
-    bool have_k1, zone;
+    bool zone;
 };
 
 // FP64 reciprocal and reciprocal square root without the long-latency IEEE sequences: the FP32
@@ -532,9 +566,32 @@ __device__ __forceinline__ bool ray_start_mixed(RayRun<Mixed>& ry, const Camera&
     ry.tau = 1.0f;
     ry.step = 0;
     ry.attempt = 0;
-    ry.have_k1 = false;
     ry.zone = false;
     return run;
+}
+
+template <bool COUNT>
+__device__ __forceinline__ void ray_prepare_mixed(RayRun<Mixed>& ry, const Scene& sc, Tally& tl) {
+#pragma unroll
+    for (int c = 0; c < 6; ++c) opaque(ry.s[c]);
+    const float rc = ks_radius<float>(ry.s[0], ry.s[1], ry.s[2], sc.aa);
+    ry.tol = step_tolerance_at<float, 1>(rc, ry.s, sc);
+    ry.zone = rc < sc.zone_r;
+    hamilton_rhs<float, true>(ry.s, (float)ry.pt, sc.a, sc.aa, sc.M, ry.k1);
+    if (COUNT) tl.rhs++;
+}
+
+template <bool COUNT>
+__device__ __forceinline__ void ray_sky_mixed(RayRun<Mixed>& ry, const Scene& sc, Tally& tl) {
+    using O = Ops<float>;
+    float ke[6];
+    hamilton_rhs<float, true>(ry.s, (float)ry.pt, sc.a, sc.aa, sc.M, ke);
+    if (COUNT) tl.rhs++;
+    const float inv = O::rsq(ke[0] * ke[0] + ke[1] * ke[1] + ke[2] * ke[2]);
+    const float sky = sky_value<float>(ke[0] * inv, ke[1] * inv, ke[2] * inv, ry.tau, sc);
+    ry.col[0] += sky;
+    ry.col[1] += sky;
+    ry.col[2] += sky;
 }
 
 // Disk crossing of a mixed-precision step.  Kept out of line: it runs on few steps and would
@@ -569,25 +626,15 @@ static __device__ __noinline__ void shade_mixed(const float (*q)[6], float h, fl
     shade_hit<float, 1>(hit, (float)ptd, (float)ktd, ct, ct[3], sc, err, tl);
 }
 
-template <int MODE, bool COUNT>
-__device__ __forceinline__ bool ray_advance_mixed(RayRun<Mixed>& ry, const Scene& sc, uint32_t* err,
-                                                  Tally& tl) {
+template <int MODE, bool COUNT, bool TOGETHER>
+__device__ __forceinline__ int ray_advance_mixed(RayRun<Mixed>& ry, const Scene& sc, uint32_t* err,
+                                                 Tally& tl, int state) {
     constexpr bool EXACT = true;
     using O = Ops<float>;
     using C = DP<float>;
     using CD = DP<double>;
     const float a = sc.a, aa = sc.aa, M = sc.M;
     const float pt = (float)ry.pt;
-    if (ry.attempt == 0 && ry.step == 0) {  // later steps: set by the commit of the step before
-        const float rc = ks_radius<float>(ry.s[0], ry.s[1], ry.s[2], aa);
-        ry.tol = step_tolerance_at<float, 1>(rc, ry.s, sc);
-        ry.zone = rc < sc.zone_r;
-    }
-    if (!ry.have_k1) {
-        hamilton_rhs<float, EXACT>(ry.s, pt, a, aa, M, ry.k1);
-        ry.have_k1 = true;
-        if (COUNT) tl.rhs++;
-    }
     const float h = ry.h;
     const float* s = ry.s;
     const float* k1 = ry.k1;
@@ -616,7 +663,8 @@ __device__ __forceinline__ bool ray_advance_mixed(RayRun<Mixed>& ry, const Scene
     }
     hamilton_rhs<float, EXACT>(nx, pt, a, aa, M, k7);
     float errv;
-    if (COUNT && ry.zone) tl.fp64++;
+    const bool going = !TOGETHER || state == kRayGoing;
+    if (COUNT && ry.zone && going) tl.fp64++;
     if (ry.zone && sc.zone_err64) {
         double em = 0.0;
         bool any = false;
@@ -646,11 +694,12 @@ __device__ __forceinline__ bool ray_advance_mixed(RayRun<Mixed>& ry, const Scene
     const bool ok = errv <= 1.0f;
     ry.h = h * 0.9f * O::powr(errv, -0.2f);
     ry.attempt++;
-    if (COUNT) {
+    if (COUNT && going) {
         tl.attempts++;
         tl.rhs += 6;
     }
-    if (!ok && ry.attempt < sc.max_attempts) return false;
+    if (TOGETHER && !going) return state;
+    if (!ok && ry.attempt < sc.max_attempts) return kRayGoing;
 
     float prev[6], prev_lo[6];
 #pragma unroll
@@ -684,10 +733,10 @@ __device__ __forceinline__ bool ray_advance_mixed(RayRun<Mixed>& ry, const Scene
     if (COUNT) tl.steps++;
     if (O::isnanr(ry.s[1])) {
         if (COUNT) tl.frozen = 1;
-        if (!sc.keep_frozen) return true;
+        if (!sc.keep_frozen) return kRayDone;
     }
     const float r_now = ks_radius<float>(ry.s[0], ry.s[1], ry.s[2], aa);
-    if (inside_horizon<float>(r_now, sc)) return true;
+    if (inside_horizon<float>(r_now, sc)) return kRayDone;
     bool near_disk = false;
     float tc = 0.5f;
     if ((prev[1] < 0.0f && ry.s[1] >= 0.0f) || (prev[1] > 0.0f && ry.s[1] <= 0.0f)) {
@@ -733,31 +782,23 @@ __device__ __forceinline__ bool ray_advance_mixed(RayRun<Mixed>& ry, const Scene
         ry.col[2] = ct[2];
         ry.tau = ct[3];
     }
+    if (beyond_escape<float>(r_now, sc)) {
+        if (TOGETHER) return kRayEscaped;
+        ray_sky_mixed<COUNT>(ry, sc, tl);
+        return kRayDone;
+    }
+    ry.step++;
+    if (!(ry.step < sc.max_steps && ry.tau > sc.cutoff_gt)) return kRayDone;
+    ry.tol = step_tolerance_at<float, 1>(r_now, ry.s, sc);
+    ry.zone = r_now < sc.zone_r;
     if (ok) {
 #pragma unroll
         for (int c = 0; c < 6; ++c) ry.k1[c] = k7[c];
-        ry.have_k1 = true;
-    } else {
-        ry.have_k1 = false;
-    }
-    if (beyond_escape<float>(r_now, sc)) {
-        float ke[6];
-        hamilton_rhs<float, EXACT>(ry.s, pt, a, aa, M, ke);
+    } else {  // a forced commit: the right-hand side at the compensated state
+        hamilton_rhs<float, EXACT>(ry.s, pt, a, aa, M, ry.k1);
         if (COUNT) tl.rhs++;
-        const float inv = O::rsq(ke[0] * ke[0] + ke[1] * ke[1] + ke[2] * ke[2]);
-        const float sky = sky_value<float>(ke[0] * inv, ke[1] * inv, ke[2] * inv, ry.tau, sc);
-        ry.col[0] += sky;
-        ry.col[1] += sky;
-        ry.col[2] += sky;
-        return true;
     }
-    ry.step++;
-    const bool done = !(ry.step < sc.max_steps && ry.tau > sc.cutoff_gt);
-    if (!done) {
-        ry.tol = step_tolerance_at<float, 1>(r_now, ry.s, sc);
-        ry.zone = r_now < sc.zone_r;
-    }
-    return done;
+    return kRayGoing;
 }
 
 // Uniform entry points used by the kernels for every arithmetic type.
@@ -771,12 +812,48 @@ __device__ __forceinline__ bool start(RayRun<Mixed>& ry, const Camera& cam, cons
     return ray_start_mixed(ry, cam, dir, sc, later_sample);
 }
 template <int MODE, bool COUNT, class R>
-__device__ __forceinline__ bool advance(RayRun<R>& ry, const Scene& sc, uint32_t* err, Tally& tl) {
-    return ray_advance<R, MODE, COUNT>(ry, sc, err, tl);
+__device__ __forceinline__ void prepare(RayRun<R>& ry, const Scene& sc, Tally& tl) {
+    ray_prepare<R, MODE, COUNT>(ry, sc, tl);
 }
 template <int MODE, bool COUNT>
-__device__ __forceinline__ bool advance(RayRun<Mixed>& ry, const Scene& sc, uint32_t* err, Tally& tl) {
-    return ray_advance_mixed<MODE, COUNT>(ry, sc, err, tl);
+__device__ __forceinline__ void prepare(RayRun<Mixed>& ry, const Scene& sc, Tally& tl) {
+    ray_prepare_mixed<COUNT>(ry, sc, tl);
+}
+template <int MODE, bool COUNT, bool TOGETHER = false, class R>
+__device__ __forceinline__ int advance(RayRun<R>& ry, const Scene& sc, uint32_t* err, Tally& tl,
+                                       int state = kRayGoing) {
+    return ray_advance<R, MODE, COUNT, TOGETHER>(ry, sc, err, tl, state);
+}
+template <int MODE, bool COUNT, bool TOGETHER = false>
+__device__ __forceinline__ int advance(RayRun<Mixed>& ry, const Scene& sc, uint32_t* err, Tally& tl,
+                                       int state = kRayGoing) {
+    return ray_advance_mixed<MODE, COUNT, TOGETHER>(ry, sc, err, tl, state);
+}
+template <int MODE, bool COUNT, class R>
+__device__ __forceinline__ void sky(RayRun<R>& ry, const Scene& sc, Tally& tl) {
+    ray_sky<R, MODE, COUNT>(ry, sc, tl);
+}
+template <int MODE, bool COUNT>
+__device__ __forceinline__ void sky(RayRun<Mixed>& ry, const Scene& sc, Tally& tl) {
+    ray_sky_mixed<COUNT>(ry, sc, tl);
+}
+
+// Runs the rays of a warp to their ends.  TOGETHER: all 32 lanes call (a lane without a ray passes
+// active = false), a vote at each attempt keeps them in step, ended ones included, and the sky is
+// added once the last ray has ended.
+template <int MODE, bool COUNT, bool TOGETHER, class R>
+__device__ __forceinline__ void run_rays(bool active, RayRun<R>& ry, const Scene& sc, uint32_t* err,
+                                         Tally& tl) {
+    if constexpr (TOGETHER) {
+        int state = active ? kRayGoing : kRayDone;
+        if (active) prepare<MODE, COUNT>(ry, sc, tl);
+        while (__any_sync(0xffffffffu, state == kRayGoing)) state = advance<MODE, COUNT, true>(ry, sc, err, tl, state);
+        if (state == kRayEscaped) sky<MODE, COUNT>(ry, sc, tl);
+    } else if (active) {
+        prepare<MODE, COUNT>(ry, sc, tl);
+        while (advance<MODE, COUNT>(ry, sc, err, tl) == kRayGoing) {
+        }
+    }
 }
 
 }  // namespace ktd

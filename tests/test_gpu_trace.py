@@ -255,10 +255,11 @@ def test_keep_frozen_rays_is_bit_identical(cuda, schedule):
 
 
 @pytest.mark.parametrize("size,spp", [((1, 1), 1), ((17, 33), 1), ((257, 15), 1), ((96, 64), 3), ((31, 7), 8),
-                                      ((48, 20), 17), ((9, 5), 33)])
+                                      ((48, 20), 17), ((9, 5), 33), ((400, 240), 1)])
 def test_persistent_units_match_plain(cuda, size, spp):
     """The persistent schedule's units (whole 16x16 tiles, several lanes per pixel at spp > 1, more
-    samples than lanes) give the plain schedule's image on the t1 view, bit for bit."""
+    samples than lanes; up to one unit per resident warp, and more) give the plain schedule's image
+    on the t1 view, bit for bit."""
     cfg, cam = workloads.scene("t1")
     cfg = workloads.scaled(cfg, *size)
     cfg.spp = spp
