@@ -8,7 +8,8 @@
 //              shape; 128-thread blocks may ask for more resident blocks per SM, which caps
 //              registers per thread)
 //   wavefront  persistent blocks of 128 threads; warps take units of 32 rays from a device
-//              work counter (resident blocks per SM)
+//              work counter (resident blocks per SM; the refill values of the list run the
+//              same kernel)
 // each in tile order and in long-rays-first order.  Every candidate must reproduce the first
 // candidate's image bit for bit (they run the same per-ray arithmetic; a device kernel counts
 // differing pixels).  Each is timed with CUDA events on the caller's stream, `reps` launches
@@ -47,6 +48,7 @@ kt_tuning make(int schedule, int bx, int by, int bps, int refill, int order, int
 std::vector<kt_tuning> default_candidates(int precision, int mode, int keep_frozen) {
     static const int kPlain[][2] = {{16, 16}, {32, 8}, {8, 8}, {16, 8}, {32, 4}, {8, 16}};
     static const int kPlain128[][2] = {{16, 8}, {8, 16}, {32, 4}};
+    static const int kRefill[] = {1, 4, 8, 16};
     std::vector<kt_tuning> out;
     for (int order : {KT_ORDER_TILES, KT_ORDER_LONG_FIRST}) {
         for (const auto& b : kPlain) out.push_back(make(KT_SCHED_PLAIN, b[0], b[1], 4, 1, order, keep_frozen));
@@ -57,7 +59,8 @@ std::vector<kt_tuning> default_candidates(int precision, int mode, int keep_froz
         // only the FP32 reference-semantics wavefront kernel has the 3/5/6 blocks-per-SM variants
         const std::vector<int> bps = (precision == KT_PREC_FP32 && mode == KT_MODE_REF) ? std::vector<int>{3, 4, 5, 6}
                                                                                        : std::vector<int>{4};
-        for (int b : bps) out.push_back(make(KT_SCHED_WAVEFRONT, 0, 0, b, 1, order, keep_frozen));
+        for (int b : bps)
+            for (int r : kRefill) out.push_back(make(KT_SCHED_WAVEFRONT, 0, 0, b, r, order, keep_frozen));
     }
     return out;
 }
