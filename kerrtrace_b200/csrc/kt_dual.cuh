@@ -123,6 +123,7 @@ struct Ops<Dual<R, N>> {
         for (int i = 0; i < N; ++i) r.d[i] = a.d[i] * b.v + a.v * b.d[i] + c.d[i];
         return r;
     }
+    static __device__ __forceinline__ D inv(const D& b) { return fdiv(D(R(1)), b); }
     // d(x^-1/2) = -1/2 x^-3/2 dx
     static __device__ __forceinline__ D rsq(const D& x) {
         D r;

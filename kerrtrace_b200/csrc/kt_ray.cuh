@@ -165,7 +165,7 @@ __device__ __forceinline__ R step_tolerance_at(R rc, const R* s, const Scene& sc
     const R aa = sc_aa<R>(sc), M = sc_M<R>(sc);
     const R rc2 = rc * rc;
     const R denH = O::fma(rc2, rc2, aa * s[1] * s[1]);
-    const R Hk = M * rc * rc2 * O::fdiv(R(1), denH);
+    const R Hk = M * rc * rc2 * O::inv(denH);
     R t = O::fdiv(Hk - lit<R>(0.05f, 0.05), lit<R>(0.3f, 0.3) - lit<R>(0.05f, 0.05));
     t = O::minr(O::maxr(t, R(0)), R(1));
     const R base = sc_tol<R>(sc);
@@ -410,10 +410,20 @@ __device__ __forceinline__ int ray_advance(RayRun<R>& ry, const Scene& sc, uint3
 #pragma unroll
     for (int c = 0; c < 6; ++c) {
         const R scale = ry.tol * O::maxr(O::absr(s[c]), R(1));
-        e[c] = O::absr(h * (C::e1 * k1[c] + C::e3 * k3[c] + C::e4 * k4[c] + C::e5 * k5[c] +
-                            C::e6 * k6[c] + C::e7 * k7[c])) / scale;
+        e[c] = O::ratio(O::absr(h * (C::e1 * k1[c] + C::e3 * k3[c] + C::e4 * k4[c] + C::e5 * k5[c] +
+                                     C::e6 * k6[c] + C::e7 * k7[c])), scale);
     }
-    const R errv = O::maxr(O::maxr(O::maxr(e[0], e[1]), O::maxr(e[2], e[3])), O::maxr(e[4], e[5]));
+    R errv = O::maxr(O::maxr(O::maxr(e[0], e[1]), O::maxr(e[2], e[3])), O::maxr(e[4], e[5]));
+    if constexpr (std::is_same<R, double>::value) {
+        if (O::isnanr(errv)) {  // a zero tolerance or an infinite state: ratio() does not cover them
+#pragma unroll
+            for (int c = 0; c < 6; ++c) {
+                const R ec = O::absr(h * (C::e1 * k1[c] + C::e3 * k3[c] + C::e4 * k4[c] + C::e5 * k5[c] +
+                                          C::e6 * k6[c] + C::e7 * k7[c]));
+                errv = O::maxr(errv, ec / (ry.tol * O::maxr(O::absr(s[c]), R(1))));
+            }
+        }
+    }
     const bool ok = errv <= R(1);
     ry.h = h * lit<R>(0.9f, 0.9) * O::powr(errv, lit<R>(-0.2f, -0.2));
     ry.attempt++;
