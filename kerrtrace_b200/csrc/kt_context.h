@@ -21,5 +21,6 @@ struct kt_context {
     unsigned long long* counters = nullptr; // 6 x u64 for the counting launches
     unsigned* order = nullptr;              // pixel order (allocated when a tuning asks for it)
     float4* bloom_scratch = nullptr;        // kt_post_fused's bloom buffer (when bloom is active)
+    float* post_tables = nullptr;           // the blur's weights and their sums
     int block_x = 16, block_y = 16;
 };

@@ -470,6 +470,7 @@ void destroy_ctx(kt_context* c) {
     cudaFree(c->counters);
     cudaFree(c->order);
     cudaFree(c->bloom_scratch);
+    cudaFree(c->post_tables);
     cudaSetDevice(prev);
     delete c;
 }
@@ -685,8 +686,13 @@ kt_status create_impl(const kt_config* cfg, int device, const float* bb_in, cons
     if ((e = cudaMalloc(&c->queue, 64)) != cudaSuccess ||
         (e = cudaMalloc(&c->counters, 8 * sizeof(unsigned long long))) != cudaSuccess ||
         (c->post.active &&
-         (e = cudaMalloc(&c->bloom_scratch, (size_t)cfg->width * cfg->height * sizeof(float4))) != cudaSuccess))
+         (e = cudaMalloc(&c->bloom_scratch, ktd::post_scratch_bytes((int)cfg->width, (int)cfg->height))) != cudaSuccess) ||
+        (e = cudaMalloc(&c->post_tables, ktd::post_table_floats(c->post) * sizeof(float) + 16)) != cudaSuccess)
         return step(cuda_fail(e, "context allocation"));
+    // the tables are complete before the context is handed out: its calls may come on any stream
+    if ((e = ktd::launch_post_tables(c->post, c->post_tables, nullptr)) != cudaSuccess ||
+        (e = cudaStreamSynchronize(nullptr)) != cudaSuccess)
+        return step(cuda_fail(e, "blur tables"));
     if ((st = step(fill_scene(c))) != KT_OK) return st;
     cudaSetDevice(prev);
     *out = c;

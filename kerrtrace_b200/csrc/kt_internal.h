@@ -17,6 +17,10 @@ struct PostParams {
     int active;       // enabled && radius > 0 && intensity > 0
     int mode;         // stated-physics luminance threshold when 1
     float threshold;
+    // device tables of the blur (launch_post_tables; also when bloom is inactive, for the separate passes)
+    const float2* weights;    // 2 radius + 1 tap weights, each twice, and a zero
+    const float* inv_wsum_x;  // per column, per row: 1 / the sum of the in-image weights
+    const float* inv_wsum_y;
 };
 
 // Tuning of the persistent tracer: resident blocks per SM (3..6 for the FP32 reference
@@ -76,7 +80,12 @@ cudaError_t launch_bloom_horizontal(const PostParams& pp, const float4* hdr, flo
                                     cudaStream_t stream);
 cudaError_t launch_post_process(const PostParams& pp, const float4* hdr, const float4* bloom,
                                 uint32_t* image, cudaStream_t stream);
-// Both post passes; scratch: a width x height float4 bloom buffer (unused when bloom is off).
+// Fills pp's tables (post_table_floats(pp) floats of device memory at `tables`) on `stream`.
+size_t post_table_floats(const PostParams& pp);
+cudaError_t launch_post_tables(PostParams& pp, float* tables, cudaStream_t stream);
+// Both post passes; scratch: post_scratch_bytes(width, height) of device memory for the bloom buffer
+// (unused when bloom is off).
+size_t post_scratch_bytes(int width, int height);
 cudaError_t launch_post_fused(const PostParams& pp, const float4* hdr, uint32_t* image, float4* scratch,
                               cudaStream_t stream);
 // FP32 FMA throughput probe: `blocks` x 512 threads, each running 8 independent FMA chains of

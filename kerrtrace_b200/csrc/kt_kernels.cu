@@ -10,17 +10,17 @@
 //   trace_wavefront_kernel  persistent: one block per resident slot, each warp takes units of 32
 //                           rays (pixels x samples) from a device work counter.
 // Post kernels (replace bloom_horizontal / post_process, cuda/kernel.cu:144-251):
-//   bloom_h_kernel          horizontal normalised Gaussian, register-blocked over staged rows
-//   post_v_kernel           vertical Gaussian streamed from the bloom buffer + composite, ACES,
-//                           sRGB OETF, 0x00RRGGBB pack
-//   post_vt_kernel          the same over the column-major bloom buffer of the fused post
+//   bloom_h_kernel          horizontal normalised Gaussian over tiles staged in pairs of rows
+//   post_v_kernel           vertical Gaussian over tiles staged in pairs of columns + composite,
+//                           ACES, sRGB OETF, 0x00RRGGBB pack
 //   tonemap_kernel          tone map alone (bloom inactive)
-// kt_post_fused runs both passes over a bloom buffer that the context owns, stored column-major
-// between them: bloom_h_kernel<true> writes it, post_vt_kernel stages its columns like rows.  The post kernels
-// produce the reference's bits: same tap order, weights, division and tone-map expressions.
+// kt_post_fused runs both passes over a bloom buffer that the context owns, laid out as the vertical
+// pass stages it.  The post kernels produce the reference's bits: same tap order, weights, division
+// and tone-map expressions.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
 #include <type_traits>
 
 #include "kt_internal.h"
@@ -610,12 +610,15 @@ __device__ __forceinline__ float srgb1(float x) {
     if (x <= 0.0031308f) return 12.92f * x;
     return 1.055f * powf(x, 0.4166666666666667f) - 0.055f;
 }
+// Nearest integer of saturate(v) x 255 in the low byte: adding 3 x 2^22 leaves no fraction bits, so the
+// addition rounds as the conversion instruction does, on the FMA pipe instead of the conversion unit.
 __device__ __forceinline__ uint32_t to_byte(float v) {
-    return (uint32_t)(unsigned char)__float2int_rn(__saturatef(v) * 255.0f);
+    return __float_as_uint(__fadd_rn(__fmul_rn(__saturatef(v), 255.0f), 12582912.0f));
 }
 __device__ __forceinline__ uint32_t tone_pack(float r, float g, float b) {
     const float mr = srgb1(aces1(r)), mg = srgb1(aces1(g)), mb = srgb1(aces1(b));
-    return (to_byte(mr) << 16) | (to_byte(mg) << 8) | to_byte(mb);
+    // bytes b, g, r and the zero above r's
+    return __byte_perm(__byte_perm(to_byte(mb), to_byte(mg), 0x0040), to_byte(mr), 0x5410);
 }
 
 // Bloom source (stated physics: only the part of the luminance above the threshold blooms).
@@ -626,378 +629,527 @@ __device__ __forceinline__ float4 bloom_source(float4 c, const PostParams& pp) {
     return make_float4(c.x * k, c.y * k, c.z * k, c.w);
 }
 
-// ---- separable Gaussian, register-blocked ------------------------------------------------
-// Each thread makes kBJ consecutive outputs along the blur direction from one stream of
-// kBJ + 2R source values: value k feeds output j with weight w[k - j] (tap i = k - j - R), so
-// every output still accumulates its taps in increasing i, the order of the reference's loop
-// (cuda/kernel.cu:156-166, 199-209), with the same contracted multiply-adds, and gets the same
-// bits.  A source value is read once per kBJ outputs instead of once per output.  The weight
-// sum of an output (its in-image weights, added in the same order) depends only on its position
-// and is computed once per block.  Chunks whose taps all lie inside the image run the head /
-// middle / tail loop; chunks at the border run the reference's per-output loop.
-constexpr int kBJ = 8;
+// ---- separable Gaussian on pairs of lines -------------------------------------------------
+// A blur line is a row (horizontal pass) or a column (vertical pass).  A block blurs kTPairs pairs of
+// lines over kTPos positions: its sources are staged in shared memory with the two lines of a pair
+// side by side, (r0, r1, g0, g1) and (b0, b1), so that one packed multiply-add (fma.f32x2) makes a
+// tap of both lines.  Each thread makes kBJ consecutive outputs of one pair from one stream of
+// kBJ + 2R values: value k feeds output j with weight w[k - j] (tap i = k - j - R), so every output
+// still accumulates its taps in increasing i, the order of the reference's loop
+// (cuda/kernel.cu:156-166, 199-209), with the same single multiply-adds, and gets the same bits.
+// Taps outside the image multiply staged zeros, which leaves a sum as it is (the reference skips
+// them).
+//
+// What bounds it: the FMA pipe (3 (2R + 1) multiply-adds per pixel and pass).  A packed multiply-add
+// holds the pipe as long as two plain ones but takes one issue slot, so the loads of the taps, the
+// staging and the tone map (as many instructions as the blur itself at R = 24) go out beside it; the
+// plain multiply-adds of an earlier form competed with them for slots and kept the pipe 37% busy.
+// 64 x 32-pixel tiles of 128 threads: 43 KB and 5 blocks per SM at R = 24, 7 blocks per SM and
+// frame at 1920x1080 (1020 blocks: a 128-wide tile would leave some SMs 4 and some 3).  Both passes
+// back to back (fused): 1920x1080 R = 24 66.4 -> 45.3 us, 3840x2160 213 -> 168 us, 2100x900 R = 48 118
+// -> 68.9 us, 960x540 30.9 -> 21.0 us.  Without the blur 1920x1080 takes 31 us and without the staging 41:
+// what is left beside the multiply-adds (18 us) is each block's chain of loads, tone map and
+// stores with 16 to 20 warps per SM to cover it.
+constexpr int kBJ = 8, kTPairs = 16, kTPos = 64, kTThreads = kTPairs * (kTPos / kBJ);
+constexpr int kTWarps = kTThreads / 32;
 
-template <class Load>
-__device__ __forceinline__ void blur_interior(const Load& load, const float* w, int R, float (&acc)[kBJ][3]) {
+struct PairTile {
+    ulonglong2* rg;  // kTPairs x stride: (r0, r1), (g0, g1)
+    uint64_t* b;     // kTPairs x stride: (b0, b1)
+    uint64_t* w;     // 2R + 2: (w, w), the last one zero
+    float* inv;      // kTPos: 1 / weight sum of the tile's positions
+};
+// odd strides: the 8 (16) lanes of a shared-memory phase read different 16 (8)-byte banks
+__host__ __device__ constexpr int pair_stride(int R) { return (kTPos + 2 * R) | 1; }
+__host__ __device__ constexpr size_t pair_smem(int R) {
+    return (size_t)kTPairs * pair_stride(R) * 24 + (size_t)(2 * R + 2) * 8 + kTPos * sizeof(float);
+}
+__device__ __forceinline__ PairTile pair_tile(void* smem, int R) {
+    PairTile t;
+    t.rg = static_cast<ulonglong2*>(smem);
+    t.b = reinterpret_cast<uint64_t*>(t.rg + kTPairs * pair_stride(R));
+    t.w = t.b + kTPairs * pair_stride(R);
+    t.inv = reinterpret_cast<float*>(t.w + 2 * R + 2);
+    return t;
+}
+
+__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
+    return (uint64_t)__float_as_uint(lo) | (uint64_t)__float_as_uint(hi) << 32;
+}
+__device__ __forceinline__ float lo2(uint64_t v) { return __uint_as_float((unsigned)v); }
+__device__ __forceinline__ float hi2(uint64_t v) { return __uint_as_float((unsigned)(v >> 32)); }
+__device__ __forceinline__ void fma2(uint64_t& acc, uint64_t v, uint64_t w) {
+    asm("fma.rn.ftz.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(v), "l"(w));
+}
+__device__ __forceinline__ void tap2(uint64_t (&acc)[3], const ulonglong2& rg, uint64_t b, uint64_t w) {
+    fma2(acc[0], rg.x, w);
+    fma2(acc[1], rg.y, w);
+    fma2(acc[2], b, w);
+}
+
+// kBJ outputs of one pair; rg, b: the thread's first source.
+__device__ __forceinline__ void blur_pair(const ulonglong2* rg, const uint64_t* b, const uint64_t* w, int R,
+                                          uint64_t (&acc)[kBJ][3]) {
 #pragma unroll
-    for (int j = 0; j < kBJ; ++j) acc[j][0] = acc[j][1] = acc[j][2] = 0.0f;
+    for (int j = 0; j < kBJ; ++j) acc[j][0] = acc[j][1] = acc[j][2] = 0;
+    if (2 * R < kBJ - 1) {  // fewer taps than outputs: one output after the other
+#pragma unroll
+        for (int j = 0; j < kBJ; ++j)
+            for (int i = 0; i <= 2 * R; ++i) tap2(acc[j], rg[j + i], b[j + i], w[i]);
+        return;
+    }
+    // The last kBJ weights in registers, weight i in slot i mod kBJ: every use has a fixed slot in
+    // the unrolled steps and nothing is shifted.
+    uint64_t wr[kBJ];
+#pragma unroll
+    for (int i = 0; i < kBJ; ++i) wr[i] = w[i];
     // head: value k (< kBJ - 1) feeds outputs 0..k
 #pragma unroll
     for (int k = 0; k < kBJ - 1; ++k) {
-        const float4 v = load(k);
+        const ulonglong2 c = rg[k];
+        const uint64_t d = b[k];
 #pragma unroll
-        for (int j = 0; j <= k; ++j) {
-            const float wi = w[k - j];
-            acc[j][0] += v.x * wi;
-            acc[j][1] += v.y * wi;
-            acc[j][2] += v.z * wi;
+        for (int j = 0; j <= k; ++j) tap2(acc[j], c, d, wr[k - j]);
+    }
+    // middle: value k (kBJ - 1 .. 2R) feeds every output, in rounds of kBJ steps and a short last one
+    const int mid = 2 * R + 2 - kBJ;
+    int k0 = kBJ - 1;
+#pragma unroll 1
+    for (; k0 + kBJ <= kBJ - 1 + mid; k0 += kBJ) {
+#pragma unroll
+        for (int s = 0; s < kBJ; ++s) {
+            const ulonglong2 c = rg[k0 + s];
+            const uint64_t d = b[k0 + s];
+#pragma unroll
+            for (int j = 0; j < kBJ; ++j) tap2(acc[j], c, d, wr[(kBJ - 1 + s - j) % kBJ]);
+            wr[s] = w[k0 + s + 1];
         }
     }
-    // middle: every output; wr[j] = w[k - j] slides with k (w has a zero at index 2R + 1)
-    float wr[kBJ];
 #pragma unroll
-    for (int j = 0; j < kBJ; ++j) wr[j] = w[kBJ - 1 - j];
-#pragma unroll 8
-    for (int k = kBJ - 1; k <= 2 * R; ++k) {
-        const float4 v = load(k);
+    for (int s = 0; s < kBJ - 1; ++s) {
+        if (k0 + s > 2 * R) break;
+        const ulonglong2 c = rg[k0 + s];
+        const uint64_t d = b[k0 + s];
 #pragma unroll
-        for (int j = 0; j < kBJ; ++j) {
-            acc[j][0] += v.x * wr[j];
-            acc[j][1] += v.y * wr[j];
-            acc[j][2] += v.z * wr[j];
-        }
-#pragma unroll
-        for (int j = kBJ - 1; j > 0; --j) wr[j] = wr[j - 1];
-        wr[0] = w[k + 1];
+        for (int j = 0; j < kBJ; ++j) tap2(acc[j], c, d, wr[(kBJ - 1 + s - j) % kBJ]);
+        wr[s] = w[k0 + s + 1];
     }
-    // tail: value 2R + t feeds outputs t..kBJ-1
+    // tail: value 2R + t feeds outputs t..kBJ-1 with weights 2R - kBJ + 2 .. 2R
+#pragma unroll
+    for (int i = 0; i < kBJ - 1; ++i) wr[i] = w[2 * R + 2 - kBJ + i];
 #pragma unroll
     for (int t = 1; t < kBJ; ++t) {
-        const float4 v = load(2 * R + t);
+        const ulonglong2 c = rg[2 * R + t];
+        const uint64_t d = b[2 * R + t];
 #pragma unroll
-        for (int j = t; j < kBJ; ++j) {
-            const float wi = w[2 * R + t - j];
-            acc[j][0] += v.x * wi;
-            acc[j][1] += v.y * wi;
-            acc[j][2] += v.z * wi;
+        for (int j = t; j < kBJ; ++j) tap2(acc[j], c, d, wr[kBJ - 2 + t - j]);
+    }
+}
+
+// Four values per lane of a row pair, 32 apart, into the staged tile; `left`: values from the lane's
+// first to the end of the segment.
+__device__ __forceinline__ void store_row_pair(float4 (&u)[4], float4 (&v)[4], ulonglong2* rg, uint64_t* b, int left,
+                                               const PostParams& pp) {
+    if (pp.mode == 1) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            u[q] = bloom_source(u[q], pp);
+            v[q] = bloom_source(v[q], pp);
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        if (32 * q < left) {
+            rg[32 * q] = make_ulonglong2(pack2(u[q].x, v[q].x), pack2(u[q].y, v[q].y));
+            b[32 * q] = pack2(u[q].z, v[q].z);
+        }
+    }
+}
+__device__ __forceinline__ void load_row_pair(const float4* row, int W, float4 (&u)[4], float4 (&v)[4], int left) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        if (32 * q < left) {
+            u[q] = __ldg(row + 32 * q);
+            v[q] = __ldg(row + W + 32 * q);
         }
     }
 }
 
-// Border chunk: the reference's loop per output, out-of-image taps skipped.  pos0 = position of
-// output 0 along the blur, n = image extent along it; load(k) is only called for in-image taps.
-template <class Load>
-__device__ __forceinline__ void blur_edge(const Load& load, const float* w, int R, int pos0, int n,
-                                          float (&acc)[kBJ][3]) {
-#pragma unroll
-    for (int j = 0; j < kBJ; ++j) {
-        float ax = 0.0f, ay = 0.0f, az = 0.0f;
-        for (int i = -R; i <= R; ++i) {
-            const int sp = pos0 + j + i;
-            if (sp < 0 || sp >= n) continue;
-            const float wi = w[i + R];
-            const float4 c = load(j + i + R);
-            ax += c.x * wi;
-            ay += c.y * wi;
-            az += c.z * wi;
-        }
-        acc[j][0] = ax;
-        acc[j][1] = ay;
-        acc[j][2] = az;
-    }
+// A pair of blurred values over the sum of their in-image weights (cuda/kernel.cu:167-171, 210-214), whose
+// reciprocal the tables hold: the fast division is that product (and no division where the sum
+// is 0: the tables hold 1).
+__device__ __forceinline__ uint64_t scale2(uint64_t v, uint64_t s) {
+    uint64_t r;
+    asm("mul.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r) : "l"(v), "l"(s));
+    return r;
 }
 
-// Sum of the in-image tap weights of the output at `pos` (n = extent), in tap order.
-__device__ __forceinline__ float weight_sum(int pos, int n, const float* w, int R) {
-    float ws = 0.0f;
-    for (int i = -R; i <= R; ++i) {
-        const int sp = pos + i;
-        if (sp < 0 || sp >= n) continue;
-        ws += w[i + R];
-    }
-    return ws;
-}
-
-__device__ __forceinline__ void load_weights(float* w, int R, float sigma, int tid, int nthreads) {
-    for (int i = tid; i <= 2 * R + 1; i += nthreads) w[i] = i <= 2 * R ? tap_weight(i - R, sigma) : 0.0f;
-}
-
-// 16-byte asynchronous copy global -> shared (cp.async, L2 only); the bytes past src_bytes are
-// zero-filled and nothing is read when src_bytes is 0.  Both addresses are 16-byte aligned.
-__device__ __forceinline__ void copy16_async(float4* dst, const float4* src, int src_bytes) {
+// Asynchronous copies global -> shared (cp.async); the bytes past src_bytes are zero-filled and
+// nothing is read when src_bytes is 0.  Both addresses are aligned to the size.
+__device__ __forceinline__ void copy16_async(void* dst, const void* src, int src_bytes) {
     const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(src), "r"(src_bytes) : "memory");
 }
+__device__ __forceinline__ void copy8_async(void* dst, const void* src, int src_bytes) {
+    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(d), "l"(src), "r"(src_bytes) : "memory");
+}
 __device__ __forceinline__ void copy_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
-// Horizontal pass (bloom_horizontal, cuda/kernel.cu:144-173): a block makes a 32-row x 64-column
-// tile.  Lane = row, warp = a kBJ-column chunk, so every tap test is uniform across the warp.
-// The 32 source rows (64 + 2R columns) are staged at an odd float4 row stride (conflict-free
-// column reads): warp w copies rows w, w + kHWarps, ..., its lanes taking consecutive
-// float4 of a row (coalesced, no index division), every copy in flight before the first is
-// waited for.
-constexpr int kHRows = 32, kHWarps = 8, kHCols = kHWarps * kBJ;
-
-__host__ __device__ constexpr int bloom_h_stride(int R) { return (kHCols + 2 * R) | 1; }
-
-// Stages kHRows lines of a line-major source (line l at src + l * pitch; n_lines lines of
-// n_pos values) into `stage`: lines line0 .. line0 + kHRows - 1, positions p0 - R ..
-// p0 + kHCols + R - 1, zero outside the source.  Returns after the block's copies have landed
-// (a barrier follows).
-__device__ __forceinline__ void stage_lines(float4* stage, int stride, int segw, const float4* __restrict__ src,
-                                            size_t pitch, int n_lines, int n_pos, int line0, int p0, int R,
-                                            int tid) {
-    const int wr = tid >> 5, ln = tid & 31;
-    for (int r = wr; r < kHRows; r += kHWarps) {
-        const int gl = line0 + r;
-        const bool line_in = gl < n_lines;
-        const float4* src_line = src + (line_in ? (size_t)gl * pitch : 0);
-        for (int c = ln; c < segw; c += 32) {
-            const int gp = p0 - R + c;
-            const bool in = line_in && gp >= 0 && gp < n_pos;
-            copy16_async(stage + r * stride + c, src_line + (in ? gp : 0), in ? 16 : 0);
-        }
-    }
-    copy_async_wait_all();
+__device__ __forceinline__ void copy4_async(void* dst, const void* src, int src_bytes) {
+    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(d), "l"(src), "r"(src_bytes) : "memory");
 }
 
-// TRANSPOSED writes the bloom buffer column-major (bloom[x * height + y]): the layout that the
-// fused post's vertical pass (post_vt_kernel) stages like this pass stages its rows.  Lanes
-// being rows, it stores straight from registers; the row-major output goes back through shared
-// memory for coalesced stores.
-template <bool TRANSPOSED>
-__global__ void __launch_bounds__(kHRows * kHWarps) bloom_h_kernel(const PostParams pp,
-                                                                    const float4* __restrict__ hdr,
-                                                                    float4* __restrict__ bloom) {
-    extern __shared__ float4 smem4[];
-    const int R = pp.radius;
-    const int segw = kHCols + 2 * R, stride = bloom_h_stride(R);
-    float4* stage = smem4;                                             // kHRows x stride
-    float* w = reinterpret_cast<float*>(stage + kHRows * stride);      // 2R + 2
-    float* wsum = w + 2 * R + 2;                                       // kHCols
-    const int x0 = blockIdx.x * kHCols, y0 = blockIdx.y * kHRows;
+// Starts the copies of the weight pairs and of the positions' reciprocal sums (`inv` of `n` entries,
+// from position p0); complete after copy_async_wait_all and a barrier.
+__device__ __forceinline__ void stage_tables(const PairTile& t, const PostParams& pp, const float* inv, int p0, int n,
+                                             int tid) {
+    for (int i = tid; i < 2 * pp.radius + 2; i += kTThreads) copy8_async(t.w + i, pp.weights + i, 8);
+    if (tid < kTPos) copy4_async(t.inv + tid, inv + (p0 + tid < n ? p0 + tid : 0), p0 + tid < n ? 4 : 0);
+}
+
+// The bloom buffer of the fused post: per pair of columns one column of (r0, r1, g0, g1), and, behind
+// them, one of (b0, b1): 12 bytes per pixel in the order in which the vertical pass stages it.
+__host__ __device__ __forceinline__ size_t bloom_pairs(int width) { return ((size_t)width + 1) / 2; }
+size_t post_scratch_bytes(int width, int height) { return bloom_pairs(width) * (size_t)height * 24; }
+
+// Horizontal pass (bloom_horizontal, cuda/kernel.cu:144-173): a block makes 32 rows x 64 columns.  A
+// warp holds the 16 row pairs of two 8-column chunks.  PAIRED writes the fused post's bloom
+// buffer straight from registers (a thread's 8 columns are 4 column pairs, consecutive pairs of rows
+// consecutive in memory); the row-major output goes back through shared memory for coalesced
+// stores.
+template <bool PAIRED>
+__global__ void __launch_bounds__(kTThreads, 5) bloom_h_kernel(const PostParams pp, const float4* __restrict__ hdr,
+                                                               float4* __restrict__ bloom) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int R = pp.radius, W = pp.width, H = pp.height;
+    const int stride = pair_stride(R), segw = kTPos + 2 * R;
+    const PairTile t = pair_tile(smem_raw, R);
+    const int x0 = blockIdx.x * kTPos, y0 = blockIdx.y * (2 * kTPairs);
     const int tid = threadIdx.x;
-    load_weights(w, R, pp.sigma, tid, blockDim.x);
-    stage_lines(stage, stride, segw, hdr, (size_t)pp.width, pp.height, pp.width, y0, x0, R, tid);
-    if (pp.mode == 1) {  // stated physics: the bloom source of each in-image value, in place
-        const int wr = tid >> 5, ln = tid & 31;
-        for (int r = wr; r < kHRows; r += kHWarps) {
-            const int gy = y0 + r;
-            for (int c = ln; c < segw; c += 32) {
-                const int gx = x0 - R + c;
-                if (gy < pp.height && gx >= 0 && gx < pp.width) stage[r * stride + c] = bloom_source(stage[r * stride + c], pp);
+    stage_tables(t, pp, pp.inv_wsum_x, x0, W, tid);
+    {
+        // a warp takes 4 row pairs, 128 columns of one at a time: 8 loads in flight per lane
+        const int warp = tid >> 5, lane = tid & 31;
+        const bool inner = x0 >= R && x0 + kTPos + R <= W && y0 + 2 * kTPairs <= H;  // no source outside
+        const float4* src = hdr + (ptrdiff_t)(y0 + 2 * warp) * W + (x0 - R + lane);
+        ulonglong2* rg = t.rg + warp * stride + lane;
+        uint64_t* b = t.b + warp * stride + lane;
+        if (inner) {
+            for (int p = warp; p < kTPairs; p += kTWarps) {
+                for (int c0 = 0; c0 < segw; c0 += 128) {
+                    float4 u[4], v[4];
+                    load_row_pair(src + c0, W, u, v, segw - c0 - lane);
+                    store_row_pair(u, v, rg + c0, b + c0, segw - c0 - lane, pp);
+                }
+                src += (size_t)2 * kTWarps * W;
+                rg += kTWarps * stride;
+                b += kTWarps * stride;
+            }
+        } else {
+            for (int p = warp; p < kTPairs; p += kTWarps) {
+                const int y = y0 + 2 * p;
+                for (int c0 = 0; c0 < segw; c0 += 128) {
+                    float4 u[4], v[4];
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const int c = c0 + 32 * q, x = x0 - R + lane + c;
+                        const bool in = x >= 0 && x < W && lane + c < segw;
+                        u[q] = in && y < H ? __ldg(src + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+                        v[q] = in && y + 1 < H ? __ldg(src + W + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    }
+                    store_row_pair(u, v, rg + c0, b + c0, segw - c0 - lane, pp);
+                }
+                src += (size_t)2 * kTWarps * W;
+                rg += kTWarps * stride;
+                b += kTWarps * stride;
             }
         }
+        copy_async_wait_all();
     }
     __syncthreads();
-    if (tid < kHCols) wsum[tid] = weight_sum(x0 + tid, pp.width, w, R);
-    const int lane = tid & 31, cb = (tid >> 5) * kBJ;
-    const float4* row = stage + lane * stride + cb;
-    auto load = [row](int k) { return row[k]; };
-    float acc[kBJ][3];
-    const int xs = x0 + cb;
-    if (2 * R >= kBJ - 1 && xs - R >= 0 && xs + kBJ - 1 + R < pp.width)
-        blur_interior(load, w, R, acc);
-    else
-        blur_edge(load, w, R, xs, pp.width, acc);
-    __syncthreads();  // staged sources no longer read; wsum written
-    if (TRANSPOSED) {  // lane = row: each output column's 32 rows are one coalesced store
-        const int gy = y0 + lane;
-        if (gy >= pp.height) return;
+    const int p = tid & (kTPairs - 1), cb = (tid / kTPairs) * kBJ;
+    uint64_t acc[kBJ][3];
+    blur_pair(t.rg + p * stride + cb, t.b + p * stride + cb, t.w, R, acc);
+    const int xs = x0 + cb, y = y0 + 2 * p;
 #pragma unroll
-        for (int j = 0; j < kBJ; ++j) {
-            const int gx = xs + j;
-            if (gx >= pp.width) break;
-            const float ws = wsum[cb + j];
-            float ax = acc[j][0], ay = acc[j][1], az = acc[j][2];
-            if (ws > 0.0f) {
-                ax /= ws;
-                ay /= ws;
-                az /= ws;
+    for (int j = 0; j < kBJ; ++j) {
+        const float s = t.inv[cb + j];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) acc[j][c] = scale2(acc[j][c], pack2(s, s));
+    }
+    if (PAIRED) {
+        float4* rg = bloom;
+        float2* b = reinterpret_cast<float2*>(bloom + bloom_pairs(W) * H);
+#pragma unroll
+        for (int j = 0; j < kBJ; j += 2) {
+            if (xs + j >= W) break;
+            const size_t at = (size_t)((xs + j) >> 1) * H + y;
+            if (y < H) {
+                rg[at] = make_float4(lo2(acc[j][0]), lo2(acc[j + 1][0]), lo2(acc[j][1]), lo2(acc[j + 1][1]));
+                b[at] = make_float2(lo2(acc[j][2]), lo2(acc[j + 1][2]));
             }
-            bloom[(size_t)gx * pp.height + gy] = make_float4(ax, ay, az, 0.0f);
+            if (y + 1 < H) {
+                rg[at + 1] = make_float4(hi2(acc[j][0]), hi2(acc[j + 1][0]), hi2(acc[j][1]), hi2(acc[j + 1][1]));
+                b[at + 1] = make_float2(hi2(acc[j][2]), hi2(acc[j + 1][2]));
+            }
         }
         return;
     }
-    constexpr int ostride = kHCols + 1;
-#pragma unroll
-    for (int j = 0; j < kBJ; ++j) {
-        const float ws = wsum[cb + j];
-        float ax = acc[j][0], ay = acc[j][1], az = acc[j][2];
-        if (ws > 0.0f) {
-            ax /= ws;
-            ay /= ws;
-            az /= ws;
-        }
-        stage[lane * ostride + cb + j] = make_float4(ax, ay, az, 0.0f);
-    }
+    // 2 x kTPairs rows of kTPos float4 (odd stride): no more than the staged sources took
     __syncthreads();
-    for (int j = tid; j < kHRows * kHCols; j += blockDim.x) {
-        const int r = j / kHCols, c = j - r * kHCols;
-        const int gy = y0 + r, gx = x0 + c;
-        if (gy < pp.height && gx < pp.width) bloom[(size_t)gy * pp.width + gx] = stage[r * ostride + c];
+    constexpr int ostride = kTPos + 1;
+    float4* out = reinterpret_cast<float4*>(smem_raw);
+    for (int half = 0; half < 2; ++half) {
+#pragma unroll
+        for (int j = 0; j < kBJ; ++j)
+            out[p * ostride + cb + j] = half ? make_float4(hi2(acc[j][0]), hi2(acc[j][1]), hi2(acc[j][2]), 0.0f)
+                                             : make_float4(lo2(acc[j][0]), lo2(acc[j][1]), lo2(acc[j][2]), 0.0f);
+        __syncthreads();
+        for (int i = tid; i < kTPairs * kTPos; i += kTThreads) {
+            const int r = i / kTPos, c = i - r * kTPos;
+            const int gy = y0 + 2 * r + half, gx = x0 + c;
+            if (gy < H && gx < W) bloom[(size_t)gy * W + gx] = out[r * ostride + c];
+        }
+        __syncthreads();
     }
 }
 
-// Vertical pass + composite + ACES + sRGB + pack (post_process, cuda/kernel.cu:175-251): a block
-// makes a 64-column x 32-row tile; warp w covers 32 columns ((w & 1) * 32) and kBJ rows
-// ((w >> 1) * kBJ); each thread streams its column of the bloom buffer with coalesced loads.
-constexpr int kVCols = 64, kVRows = 32, kVThreads = 256;
-
-__global__ void __launch_bounds__(kVThreads) post_v_kernel(const PostParams pp,
-                                                            const float4* __restrict__ hdr,
-                                                            const float4* __restrict__ bloom,
-                                                            uint32_t* __restrict__ image) {
-    extern __shared__ float smemf[];
-    const int R = pp.active ? pp.radius : 0;
-    float* w = smemf;                 // 2R + 2
-    float* wsum = w + 2 * R + 2;      // kVRows
+// Vertical pass + composite + ACES + sRGB + pack (post_process, cuda/kernel.cu:175-251): a block makes
+// 32 columns x 64 rows; a warp holds the 16 column pairs of two 8-row chunks.  PAIRED stages the
+// fused post's bloom buffer by cp.async; otherwise the row-major buffer of bloom_horizontal is
+// paired on the way in.
+template <bool PAIRED>
+__global__ void __launch_bounds__(kTThreads, 4) post_v_kernel(const PostParams pp, const float4* __restrict__ hdr,
+                                                              const float4* __restrict__ bloom,
+                                                              uint32_t* __restrict__ image) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int R = pp.radius, W = pp.width, H = pp.height;
+    const int stride = pair_stride(R), segw = kTPos + 2 * R;
+    const PairTile t = pair_tile(smem_raw, R);
+    const int x0 = blockIdx.x * (2 * kTPairs), y0 = blockIdx.y * kTPos;
     const int tid = threadIdx.x;
-    const int x0 = blockIdx.x * kVCols, y0 = blockIdx.y * kVRows;
-    if (pp.active) {
-        load_weights(w, R, pp.sigma, tid, blockDim.x);
-        __syncthreads();
-        if (tid < kVRows) wsum[tid] = weight_sum(y0 + tid, pp.height, w, R);
-        __syncthreads();
-    }
-    const int lane = tid & 31, warp = tid >> 5;
-    const int x = x0 + (warp & 1) * 32 + lane;
-    const int rb = (warp >> 1) * kBJ;
-    const int yb = y0 + rb;
-    if (x >= pp.width || yb >= pp.height) return;
-    float acc[kBJ][3];
-    if (pp.active) {
-        const float4* col = bloom + x;
-        const int W = pp.width;
-        auto load = [col, yb, R, W](int k) { return __ldg(col + (size_t)(yb - R + k) * W); };
-        if (2 * R >= kBJ - 1 && yb - R >= 0 && yb + kBJ - 1 + R < pp.height)
-            blur_interior(load, w, R, acc);
-        else
-            blur_edge(load, w, R, yb, pp.height, acc);
-    }
-#pragma unroll
-    for (int j = 0; j < kBJ; ++j) {
-        const int y = yb + j;
-        if (y >= pp.height) break;
-        const size_t idx = (size_t)y * pp.width + x;
-        const float4 base = __ldg(hdr + idx);
-        float fr = base.x, fg = base.y, fb = base.z;
-        if (pp.active) {
-            const float ws = wsum[rb + j];
-            float ax = acc[j][0], ay = acc[j][1], az = acc[j][2];
-            if (ws > 0.0f) {
-                ax /= ws;
-                ay /= ws;
-                az /= ws;
+    stage_tables(t, pp, pp.inv_wsum_y, y0, H, tid);
+    if (PAIRED) {
+        const int warp = tid >> 5, lane = tid & 31;
+        const size_t pairs = bloom_pairs(W);
+        const float2* bl = reinterpret_cast<const float2*>(bloom + pairs * H);
+        const bool inner = y0 >= R && y0 + kTPos + R <= H && x0 / 2 + kTPairs <= (int)pairs;
+        ptrdiff_t at = (ptrdiff_t)(x0 / 2 + warp) * H + (y0 - R + lane);
+        ulonglong2* rg = t.rg + warp * stride + lane;
+        uint64_t* b = t.b + warp * stride + lane;
+        for (int p = warp; p < kTPairs; p += kTWarps) {
+            if (inner) {
+#pragma unroll 4
+                for (int c = 0; c < segw - lane; c += 32) {
+                    copy16_async(rg + c, bloom + at + c, 16);
+                    copy8_async(b + c, bl + at + c, 8);
+                }
+            } else {
+                const bool line = x0 / 2 + p < (int)pairs;
+                for (int c = 0; c < segw - lane; c += 32) {
+                    const int y = y0 - R + lane + c;
+                    const bool in = line && y >= 0 && y < H;
+                    copy16_async(rg + c, in ? bloom + at + c : bloom, in ? 16 : 0);
+                    copy8_async(b + c, in ? bl + at + c : bl, in ? 8 : 0);
+                }
             }
-            fr += ax * pp.intensity;
-            fg += ay * pp.intensity;
-            fb += az * pp.intensity;
+            at += (ptrdiff_t)kTWarps * H;
+            rg += kTWarps * stride;
+            b += kTWarps * stride;
         }
-        image[idx] = tone_pack(fr, fg, fb);
+    } else {
+        const int p = tid & (kTPairs - 1), x = x0 + 2 * p;
+#pragma unroll 4
+        for (int c = tid / kTPairs; c < segw; c += kTThreads / kTPairs) {
+            const int y = y0 - R + c;
+            const bool in = y >= 0 && y < H;
+            const float4* row = bloom + (size_t)(in ? y : 0) * W;
+            float4 u = make_float4(0.f, 0.f, 0.f, 0.f), v = u;
+            if (in && x < W) u = __ldg(row + x);
+            if (in && x + 1 < W) v = __ldg(row + x + 1);
+            t.rg[p * stride + c] = make_ulonglong2(pack2(u.x, v.x), pack2(u.y, v.y));
+            t.b[p * stride + c] = pack2(u.z, v.z);
+        }
     }
-}
-
-// Vertical pass of the fused post over the column-major bloom buffer that bloom_h_kernel<true>
-// writes: a block makes a 32-column x 64-row tile.  Lane = column, warp = a kBJ-row chunk; the
-// block stages its 32 columns (64 + 2R rows each) exactly as the horizontal pass stages rows,
-// so every source value is read from L2 once per tile instead of once per kBJ outputs, then
-// blurs, composites, tone-maps and packs with the arithmetic of post_v_kernel (same bits).
-__global__ void __launch_bounds__(kHRows * kHWarps) post_vt_kernel(const PostParams pp,
-                                                                    const float4* __restrict__ hdr,
-                                                                    const float4* __restrict__ bloom_t,
-                                                                    uint32_t* __restrict__ image) {
-    extern __shared__ float4 smem4[];
-    const int R = pp.radius;
-    const int segw = kHCols + 2 * R, stride = bloom_h_stride(R);
-    float4* stage = smem4;                                             // kHRows x stride
-    float* w = reinterpret_cast<float*>(stage + kHRows * stride);      // 2R + 2
-    float* wsum = w + 2 * R + 2;                                       // kHCols
-    const int x0 = blockIdx.x * kHRows, y0 = blockIdx.y * kHCols;
-    const int tid = threadIdx.x;
-    load_weights(w, R, pp.sigma, tid, blockDim.x);
-    stage_lines(stage, stride, segw, bloom_t, (size_t)pp.height, pp.width, pp.height, x0, y0, R, tid);
+    copy_async_wait_all();
     __syncthreads();
-    if (tid < kHCols) wsum[tid] = weight_sum(y0 + tid, pp.height, w, R);
-    const int lane = tid & 31, cb = (tid >> 5) * kBJ;
-    const float4* col = stage + lane * stride + cb;
-    auto load = [col](int k) { return col[k]; };
-    float acc[kBJ][3];
-    const int ys = y0 + cb;
-    if (2 * R >= kBJ - 1 && ys - R >= 0 && ys + kBJ - 1 + R < pp.height)
-        blur_interior(load, w, R, acc);
-    else
-        blur_edge(load, w, R, ys, pp.height, acc);
-    __syncthreads();  // wsum written
-    const int x = x0 + lane;
-    if (x >= pp.width) return;
-    float4 base[kBJ];  // all of a thread's composite sources in flight before the first is used
+    const int p = tid & (kTPairs - 1), cb = (tid / kTPairs) * kBJ;
+    const int x = x0 + 2 * p, ys = y0 + cb;
+    if (x >= W || ys >= H) return;
+    const bool second = x + 1 < W;
+    uint64_t acc[kBJ][3];
+    blur_pair(t.rg + p * stride + cb, t.b + p * stride + cb, t.w, R, acc);
+    // composite sources 4 rows ahead of their tone maps
+    constexpr int kAhead = 4;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 us[kAhead], vs[kAhead];
 #pragma unroll
-    for (int j = 0; j < kBJ; ++j)
-        base[j] = ys + j < pp.height ? __ldg(hdr + (size_t)(ys + j) * pp.width + x) : make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int j = 0; j < kAhead; ++j) {
+        const float4* at = hdr + (size_t)(ys + j) * W + x;
+        us[j] = ys + j < H ? __ldg(at) : zero;
+        vs[j] = ys + j < H && second ? __ldg(at + 1) : zero;
+    }
 #pragma unroll
     for (int j = 0; j < kBJ; ++j) {
         const int y = ys + j;
-        if (y >= pp.height) break;
-        const size_t idx = (size_t)y * pp.width + x;
-        float fr = base[j].x, fg = base[j].y, fb = base[j].z;
-        const float ws = wsum[cb + j];
-        float ax = acc[j][0], ay = acc[j][1], az = acc[j][2];
-        if (ws > 0.0f) {
-            ax /= ws;
-            ay /= ws;
-            az /= ws;
+        if (y >= H) break;
+        const size_t idx = (size_t)y * W + x;
+        const float s = t.inv[cb + j];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) acc[j][c] = scale2(acc[j][c], pack2(s, s));
+        const float4 u = us[j % kAhead], v = vs[j % kAhead];
+        if (j + kAhead < kBJ) {
+            const float4* at = hdr + (size_t)(y + kAhead) * W + x;
+            us[j % kAhead] = y + kAhead < H ? __ldg(at) : zero;
+            vs[j % kAhead] = y + kAhead < H && second ? __ldg(at + 1) : zero;
         }
-        fr += ax * pp.intensity;
-        fg += ay * pp.intensity;
-        fb += az * pp.intensity;
-        image[idx] = tone_pack(fr, fg, fb);
+        image[idx] = tone_pack(u.x + lo2(acc[j][0]) * pp.intensity, u.y + lo2(acc[j][1]) * pp.intensity,
+                               u.z + lo2(acc[j][2]) * pp.intensity);
+        if (second)
+            image[idx + 1] = tone_pack(v.x + hi2(acc[j][0]) * pp.intensity, v.y + hi2(acc[j][1]) * pp.intensity,
+                                       v.z + hi2(acc[j][2]) * pp.intensity);
     }
 }
 
-// Tone map only (bloom inactive): one thread per pixel.
-__global__ void tonemap_kernel(const PostParams pp, const float4* __restrict__ hdr,
-                               uint32_t* __restrict__ image) {
+// The same from a row-major bloom buffer for radii whose tile does not fit in shared memory: one
+// pixel per thread, the reference's loop.
+__global__ void __launch_bounds__(256) post_v_wide_kernel(const PostParams pp, const float4* __restrict__ hdr,
+                                                          const float4* __restrict__ bloom,
+                                                          uint32_t* __restrict__ image) {
+    const int x = blockIdx.x * 32 + (threadIdx.x & 31), y = blockIdx.y * 8 + (threadIdx.x >> 5);
+    if (x >= pp.width || y >= pp.height) return;
+    const int R = pp.radius;
+    float ax = 0.0f, ay = 0.0f, az = 0.0f;
+    for (int i = max(-R, -y); i <= min(R, pp.height - 1 - y); ++i) {
+        const float w = __ldg(&pp.weights[i + R].x);
+        const float4 c = __ldg(bloom + (size_t)(y + i) * pp.width + x);
+        ax += c.x * w;
+        ay += c.y * w;
+        az += c.z * w;
+    }
+    const float s = __ldg(pp.inv_wsum_y + y);
+    const size_t idx = (size_t)y * pp.width + x;
+    const float4 base = __ldg(hdr + idx);
+    image[idx] = tone_pack(base.x + __fmul_rn(ax, s) * pp.intensity, base.y + __fmul_rn(ay, s) * pp.intensity,
+                           base.z + __fmul_rn(az, s) * pp.intensity);
+}
+
+// Tone map only (bloom inactive): 4 pixels per thread, their loads issued together.
+__global__ void __launch_bounds__(256) tonemap_kernel(const PostParams pp, const float4* __restrict__ hdr,
+                                                      uint32_t* __restrict__ image) {
     const size_t n = (size_t)pp.width * pp.height;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-         i += (size_t)gridDim.x * blockDim.x) {
-        const float4 c = __ldg(hdr + i);
-        image[i] = tone_pack(c.x, c.y, c.z);
-    }
+    const size_t i0 = (size_t)blockIdx.x * 1024 + threadIdx.x;
+    float4 c[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) c[k] = i0 + 256 * k < n ? __ldg(hdr + i0 + 256 * k) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+        if (i0 + 256 * k < n) image[i0 + 256 * k] = tone_pack(c[k].x, c[k].y, c[k].z);
 }
 
-static size_t bloom_h_smem(int R) {
-    return (size_t)kHRows * bloom_h_stride(R) * sizeof(float4) + (size_t)(2 * R + 2 + kHCols) * sizeof(float);
+// The blur's tables, made once per context: weight pairs 0 .. 2R (and a zero behind them), and for every
+// column and row the reciprocal of the sum of its in-image weights, added in tap order (1 where the
+// sum is 0).
+__global__ void __launch_bounds__(256) post_weights_kernel(int R, float sigma, float2* __restrict__ weights) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const float w = i <= 2 * R ? tap_weight(i - R, sigma) : 0.0f;
+    if (i <= 2 * R + 1) weights[i] = make_float2(w, w);
 }
-static size_t post_v_smem(int R) { return (size_t)(2 * R + 2 + kVRows) * sizeof(float); }
+__global__ void __launch_bounds__(256) post_weight_sums_kernel(const PostParams pp, float* __restrict__ inv_x,
+                                                               float* __restrict__ inv_y) {
+    const int R = pp.radius;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int axis = i < pp.width ? 0 : 1, pos = axis ? i - pp.width : i, n = axis ? pp.height : pp.width;
+    if (i >= pp.width + pp.height) return;
+    float ws = 0.0f;
+    for (int k = max(-R, -pos); k <= min(R, n - 1 - pos); ++k) ws += pp.weights[k + R].x;
+    (axis ? inv_y : inv_x)[pos] = ws > 0.0f ? 1.0f / ws : 1.0f;
+}
+
 constexpr size_t kSmemLimit = 200 * 1024;
+// Largest radius of the horizontal pass and the fused post (about 163).
+static bool radius_fits(int R) {
+    return (size_t)32 * ((kTPos + 2 * R) | 1) * 16 + (size_t)(2 * R + 2 + kTPos) * 4 <= kSmemLimit;
+}
 
 static cudaError_t set_smem(const void* fn, size_t bytes) {
     if (bytes <= 48 * 1024) return cudaSuccess;
     return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
+// Radii above this (25583) are refused by every post entry point and have no tables.
+static bool radius_has_tables(int R) { return ((size_t)2 * R + 2 + 32) * sizeof(float) <= kSmemLimit; }
+
+size_t post_table_floats(const PostParams& pp) {
+    return radius_has_tables(pp.radius) ? 2 * ((size_t)2 * pp.radius + 2) + pp.width + pp.height : 0;
+}
+
+cudaError_t launch_post_tables(PostParams& pp, float* tables, cudaStream_t st) {
+    if (!radius_has_tables(pp.radius)) return cudaSuccess;
+    const int nw = 2 * pp.radius + 2;
+    float2* weights = reinterpret_cast<float2*>(tables);
+    float* sums = tables + 2 * (size_t)nw;
+    pp.weights = weights;
+    pp.inv_wsum_x = sums;
+    pp.inv_wsum_y = sums + pp.width;
+    post_weights_kernel<<<(nw + 255) / 256, 256, 0, st>>>(pp.radius, pp.sigma, weights);
+    post_weight_sums_kernel<<<(pp.width + pp.height + 255) / 256, 256, 0, st>>>(pp, sums, sums + pp.width);
+    return cudaGetLastError();
+}
+
+static cudaError_t launch_tonemap(const PostParams& pp, const float4* hdr, uint32_t* image, cudaStream_t st) {
+    const size_t n = (size_t)pp.width * pp.height;
+    tonemap_kernel<<<(unsigned)((n + 1023) / 1024), 256, 0, st>>>(pp, hdr, image);
+    return cudaGetLastError();
+}
+
+template <bool PAIRED>
+static cudaError_t launch_h(const PostParams& pp, const float4* hdr, float4* bloom, cudaStream_t st) {
+    // the row-major output's transposition takes kTPairs x (kTPos + 1) float4 of the staged tile
+    const size_t sm = std::max(pair_smem(pp.radius), (size_t)kTPairs * (kTPos + 1) * 16);
+    const cudaError_t e = set_smem((const void*)bloom_h_kernel<PAIRED>, sm);
+    if (e != cudaSuccess) return e;
+    const dim3 grid((pp.width + kTPos - 1) / kTPos, (pp.height + 2 * kTPairs - 1) / (2 * kTPairs));
+    bloom_h_kernel<PAIRED><<<grid, kTThreads, sm, st>>>(pp, hdr, bloom);
+    return cudaGetLastError();
+}
+template <bool PAIRED>
+static cudaError_t launch_v(const PostParams& pp, const float4* hdr, const float4* bloom, uint32_t* image,
+                            cudaStream_t st) {
+    const size_t sm = pair_smem(pp.radius);
+    const cudaError_t e = set_smem((const void*)post_v_kernel<PAIRED>, sm);
+    if (e != cudaSuccess) return e;
+    const dim3 grid((pp.width + 2 * kTPairs - 1) / (2 * kTPairs), (pp.height + kTPos - 1) / kTPos);
+    post_v_kernel<PAIRED><<<grid, kTThreads, sm, st>>>(pp, hdr, bloom, image);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_bloom_horizontal(const PostParams& pp, const float4* hdr, float4* bloom, cudaStream_t st) {
     if (pp.width <= 0 || pp.height <= 0) return cudaSuccess;
-    const size_t sm = bloom_h_smem(pp.radius);
-    if (sm > kSmemLimit) return cudaErrorInvalidValue;
-    cudaError_t e = set_smem((const void*)bloom_h_kernel<false>, sm);
-    if (e != cudaSuccess) return e;
-    const dim3 grid((pp.width + kHCols - 1) / kHCols, (pp.height + kHRows - 1) / kHRows);
-    bloom_h_kernel<false><<<grid, kHRows * kHWarps, sm, st>>>(pp, hdr, bloom);
-    return cudaGetLastError();
+    if (!radius_fits(pp.radius)) return cudaErrorInvalidValue;
+    return launch_h<false>(pp, hdr, bloom, st);
 }
 
 cudaError_t launch_post_process(const PostParams& pp, const float4* hdr, const float4* bloom,
                                 uint32_t* image, cudaStream_t st) {
     if (pp.width <= 0 || pp.height <= 0) return cudaSuccess;
-    const size_t sm = pp.active ? post_v_smem(pp.radius) : 0;
-    if (sm > kSmemLimit) return cudaErrorInvalidValue;
-    cudaError_t e = set_smem((const void*)post_v_kernel, sm);
-    if (e != cudaSuccess) return e;
-    const dim3 grid((pp.width + kVCols - 1) / kVCols, (pp.height + kVRows - 1) / kVRows);
-    post_v_kernel<<<grid, kVThreads, sm, st>>>(pp, hdr, bloom, image);
+    if (!pp.active) return launch_tonemap(pp, hdr, image, st);
+    if (pair_smem(pp.radius) <= kSmemLimit) return launch_v<false>(pp, hdr, bloom, image, st);
+    if (!radius_has_tables(pp.radius)) return cudaErrorInvalidValue;
+    const dim3 grid((pp.width + 31) / 32, (pp.height + 7) / 8);
+    post_v_wide_kernel<<<grid, 256, 0, st>>>(pp, hdr, bloom, image);
     return cudaGetLastError();
+}
+
+cudaError_t launch_post_fused(const PostParams& pp, const float4* hdr, uint32_t* image, float4* scratch,
+                              cudaStream_t st) {
+    if (pp.width <= 0 || pp.height <= 0) return cudaSuccess;
+    if (!pp.active) return launch_tonemap(pp, hdr, image, st);
+    if (!scratch || !radius_fits(pp.radius)) return cudaErrorInvalidValue;
+    const cudaError_t e = launch_h<true>(pp, hdr, scratch, st);
+    return e != cudaSuccess ? e : launch_v<true>(pp, hdr, scratch, image, st);
 }
 
 // FP32 FMA throughput probe (the denominator of the trace's roofline): eight independent
@@ -1020,30 +1172,6 @@ __global__ void __launch_bounds__(512) fma_probe_kernel(float b, float c, int it
 
 cudaError_t launch_fma_probe(int blocks, int iters, float* sink, cudaStream_t st) {
     fma_probe_kernel<<<blocks, 512, 0, st>>>(0.999999f, 1e-6f, iters, sink);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_post_fused(const PostParams& pp, const float4* hdr, uint32_t* image, float4* scratch,
-                              cudaStream_t st) {
-    if (pp.width <= 0 || pp.height <= 0) return cudaSuccess;
-    if (!pp.active) {
-        int dev = 0, sms = 148;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        tonemap_kernel<<<sms * 8, 256, 0, st>>>(pp, hdr, image);
-        return cudaGetLastError();
-    }
-    if (!scratch) return cudaErrorInvalidValue;
-    // both passes through the context's scratch, column-major in between (never seen by callers)
-    const size_t sm = bloom_h_smem(pp.radius);
-    if (sm > kSmemLimit) return cudaErrorInvalidValue;
-    cudaError_t e = set_smem((const void*)bloom_h_kernel<true>, sm);
-    if (e == cudaSuccess) e = set_smem((const void*)post_vt_kernel, sm);
-    if (e != cudaSuccess) return e;
-    const dim3 gh((pp.width + kHCols - 1) / kHCols, (pp.height + kHRows - 1) / kHRows);
-    bloom_h_kernel<true><<<gh, kHRows * kHWarps, sm, st>>>(pp, hdr, scratch);
-    const dim3 gv((pp.width + kHRows - 1) / kHRows, (pp.height + kHCols - 1) / kHCols);
-    post_vt_kernel<<<gv, kHRows * kHWarps, sm, st>>>(pp, hdr, scratch, image);
     return cudaGetLastError();
 }
 

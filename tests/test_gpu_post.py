@@ -137,3 +137,50 @@ def test_stated_physics_bloom_threshold(cuda, orc, size, radius):
         assert not np.array_equal(img_0.cpu().numpy().view(np.uint32), i_f)
     ctx0.close()
     ctx.close()
+
+
+@pytest.mark.parametrize("size,radius", [((1, 1), 24.0), ((7, 3), 1.0), ((33, 65), 2.0), ((65, 129), 3.5), ((64, 64), 4.0),
+                                         ((63, 127), 24.0), ((1, 200), 24.0), ((200, 1), 24.0), ((641, 97), 90.0),
+                                         ((400, 60), 163.0), ((50, 40), 300.0)])
+def test_post_tiles_against_oracle(cuda, orc, size, radius):
+    """Tiles of line pairs at their edges (odd lines and positions, frames smaller than a tile, radii
+    with fewer taps than a thread's outputs and up to the largest that fits): the fused pair equals
+    the separate passes bit for bit, the bloom buffer is the double-precision horizontal Gaussian to
+    float rounding (sum of 2R + 1 products: relative error (2R + 2) 2^-24, plus the fast exponential's
+    2e-6 per weight), and the image is the oracle's to one code value.  Radius 300 is beyond the
+    tiles: only the vertical pass takes it (bloom buffer given)."""
+    cfg, _ = workloads.scene("t1")
+    cfg = workloads.scaled(cfg, *size)
+    cfg.bloom_radius = radius
+    R, sigma, active = _bloom_consts(cfg)
+    w, h = size
+    hdr = _hdr_input(cuda, cfg, 5)
+    ctx = kt.Context(cfg)
+    bloom = cuda.zeros((w * h, 4), device="cuda")
+    img_s, img_f = (cuda.zeros(w * h, dtype=cuda.int32, device="cuda") for _ in range(2))
+    src = hdr.cpu().numpy().astype(np.float64).reshape(h, w, 4)[..., :3]
+    k = np.exp(-np.arange(-R, R + 1) ** 2 / (2 * sigma ** 2))
+    full = np.zeros((h, w + 2 * R, 3))
+    full[:, R:R + w] = src
+    ones = np.zeros(w + 2 * R)
+    ones[R:R + w] = 1.0
+    exp_b = sum(k[i] * full[:, i:i + w] for i in range(2 * R + 1)) / sum(k[i] * ones[i:i + w] for i in range(2 * R + 1))[None, :, None]
+    if radius <= 163:
+        ctx.bloom_horizontal(hdr.data_ptr(), bloom.data_ptr())
+        ctx.post_fused(hdr.data_ptr(), img_f.data_ptr())
+    else:
+        with pytest.raises(kt.KtError):
+            ctx.bloom_horizontal(hdr.data_ptr(), bloom.data_ptr())
+        bloom[:, :3] = cuda.from_numpy(exp_b.reshape(-1, 3).astype(np.float32)).cuda()
+    ctx.post_process(hdr.data_ptr(), bloom.data_ptr(), img_s.data_ptr())
+    cuda.cuda.synchronize()
+    got = bloom.cpu().numpy().reshape(h, w, 4)[..., :3].astype(np.float64)
+    assert np.max(np.abs(got - exp_b) / np.maximum(np.abs(exp_b), 1e-30)) < (2 * R + 2) * 2.0 ** -24 + 4e-6
+    i_s = img_s.cpu().numpy().view(np.uint32)
+    if radius <= 163:
+        assert np.array_equal(i_s, img_f.cpu().numpy().view(np.uint32))
+    exp = orc.post(hdr.cpu().numpy(), w, h, R, sigma, cfg.bloom_intensity)
+    d = np.max(np.abs(np.stack([(i_s >> s) & 255 for s in (16, 8, 0)]).astype(int) -
+                      np.stack([(exp >> s) & 255 for s in (16, 8, 0)]).astype(int)), axis=0)
+    assert d.max() <= 1, np.bincount(d)
+    ctx.close()
