@@ -198,7 +198,7 @@ kt_status kt_generate_blackbody_lut(uint32_t size, float max_temp, float wavelen
 kt_status kt_generate_disk_lut(const kt_kerr_params* params, float disk_outer, uint32_t size,
                                float* out);
 /* The same two tables generated on the device, on `stream`, into device memory (dev_out:
- * float[4*size] / float[size]), one thread per row.  They use CUDA's accurate math functions and
+ * float[4*size] / float[size]).  They use CUDA's accurate math functions and
  * agree with the host tables to a few ulp, not bit for bit (CUDA's and glibc's libm round
  * differently in the last place).  For hosts that build many per-scene tables (batches) or keep
  * everything on the device. */

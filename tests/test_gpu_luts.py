@@ -40,6 +40,20 @@ def test_device_luts_match_host_luts(cuda, name):
     assert dev_disk[0] == 0.0 and host_disk[0] == 0.0
 
 
+@pytest.mark.parametrize("size,step", [(2, 340.0), (15, 10.0), (17, 5.3), (33, 5.4), (16, 1.0), (100, 1.7)])
+def test_device_blackbody_rows_and_chunks(cuda, size, step):
+    """Row counts around a block's and wavelength grids around a chunk's (2, 35, 65, 63, 341 and 201
+    wavelengths): the host table to the same 2e-5 of each row."""
+    host = kt.generate_blackbody_lut(size, 6e4, 380.0, 720.0, step)
+    dev = cuda.full((size + 1, 4), float("nan"), device="cuda")
+    kt.generate_blackbody_lut_device(size, 6e4, 380.0, 720.0, step, dev.data_ptr())
+    cuda.cuda.synchronize()
+    got = dev.cpu().numpy()
+    assert np.all(np.isnan(got[size]))  # nothing beyond the table
+    scale = np.maximum(np.abs(host[:, :3]).max(1, keepdims=True), 1e-37)
+    assert (np.abs(got[:size, :3].astype(np.float64) - host[:, :3]) / scale).max() < 2e-5
+
+
 @pytest.mark.parametrize("name,size", [("c2", (320, 180)), ("t1", None), ("c1", (128, 128))])
 def test_context_with_device_luts_renders_within_parity(cuda, name, size):
     """A context whose LUTs were generated on the device (kt_context_create_device_luts) renders
