@@ -158,6 +158,22 @@ __device__ __forceinline__ void rhs_vjp(const R* Y, const R* l, R pt, R a, R aa,
     dpt = -fL;
 }
 
+// The float product as a call (arguments and results in registers): seven inlined copies made the reverse
+// step 70 KB of straight code, and with two warps per scheduler a quarter of the time went to
+// instruction fetches (512x512: 444 -> 414 us).  In double the copies are the faster form (the
+// call spills around its 24 registers of arguments: 669 -> 742 us at 256x256).
+struct Vec6 {
+    float v[6];
+};
+struct VjpOut {
+    float y[6], da, dpt;
+};
+static __device__ __noinline__ VjpOut rhs_vjp_call(Vec6 Y, Vec6 l, float pt, float a, float aa, float M) {
+    VjpOut o;
+    rhs_vjp<float>(Y.v, l.v, pt, a, aa, M, o.y, o.da, o.dpt);
+    return o;
+}
+
 // Tangent slots of the shading duals.
 enum : int { kSX = 0, kSPt = 6, kSKt = 7, kSA = 8, kSTs = 9, kSRo = 10, kSN = 11 };
 
@@ -438,18 +454,20 @@ __device__ __forceinline__ R rk_a(int m, int j) {
 }
 
 // ---- forward: record / replay ----------------------------------------------------------------
-// Four resident 128-thread blocks per SM: 128 registers at most (the FP64 kernel spills about
-// 400 B there; 192 registers and two blocks otherwise).
+// Resident 128-thread blocks per SM asked of the compiler: four in FP32 (128 registers at most), three in
+// FP64 (168; with four the kernel spills 380 B: 512x512 1.14 ms against 1.03).  A warp takes an 8x4
+// patch of the frame, whose rays have more equal lengths than a row's 32 (512x512: FP32 437 -> 391
+// us with the host's tables, FP64 1.39 -> 1.14 ms).
 // RR: arithmetic type of the records (R, or float records replayed in double arithmetic).
 template <class R, bool REPLAY, class RR = R>
-__global__ void __launch_bounds__(128, 4) diff_forward_kernel(const Scene sc, const Camera cam, const CameraD camd,
+__global__ void __launch_bounds__(128, sizeof(R) == 8 ? 3 : 4) diff_forward_kernel(const Scene sc, const Camera cam, const CameraD camd,
                                                           const DiffRecRaw rec, float4* __restrict__ hdr,
                                                           double* __restrict__ hdr64, uint32_t* __restrict__ err,
                                                           uint32_t* __restrict__ flags) {
-    const unsigned n_px = (unsigned)sc.width * (unsigned)sc.height;
-    const unsigned p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= n_px) return;
-    const int px = (int)(p % (unsigned)sc.width), py = (int)(p / (unsigned)sc.width);
+    int px, py;
+    tile_to_pixel(blockIdx.x * blockDim.x + threadIdx.x, sc.width, px, py);
+    if (px >= sc.width || py >= sc.height) return;
+    const unsigned p = (unsigned)py * (unsigned)sc.width + (unsigned)px;
     RayRun<R> ry;
     Tally tl;
     tl.clear();
@@ -737,7 +755,11 @@ __global__ void __launch_bounds__(128, BackMinBlocks<R>::v) diff_backward_kernel
             while (si >= 0) {
                 const DiffSeg<RR>* sg = seg_at<RR>(rec, si);
                 const unsigned hits = sg->hits;
+                // the last segment ends with the ray's last shaded crossing: the transmittance behind it
+                // has no use, and its root and shading, at a different step of each lane, are left out
+                // (512x512: FP32 479 -> 444 us, FP64 955 -> 816)
                 const int n = first ? 32 - __clz((int)hits) : sg->n;
+                const int last_hit = first ? n - 1 : -1;
                 first = false;
                 // forward sweep: states, stages, transmittance at the shaded crossings
                 {
@@ -770,10 +792,10 @@ __global__ void __launch_bounds__(128, BackMinBlocks<R>::v) diff_backward_kernel
                             for (int c = 0; c < 6; ++c) K[j][0][c] = K7[c];
                         }
                         dp5_stages<R>(s, sg->h[j], pt, a, aa, M, K[j], nx, K7, j > 0);
-                        if (hits >> j & 1u) {
+                        if (hits >> j & 1u) TIN[j] = tau;
+                        if ((hits >> j & 1u) && j != last_hit) {
                             R X[6], c3[3], al;
                             step_hit<R>(s, nx, K[j], K7, sg->h[j], X, nullptr);
-                            TIN[j] = tau;
                             if (shade_eval<R, R>(X, pt, kt, sc, dl, c3, al)) tau *= R(1) - al;
                         }
 #pragma unroll
@@ -870,7 +892,21 @@ __global__ void __launch_bounds__(128, BackMinBlocks<R>::v) diff_backward_kernel
                         for (int c = 0; c < 6; ++c) nz = nz || acc[m][c] != R(0);
                         if (!nz) continue;
                         R lY[6], da, dpt;
-                        rhs_vjp<R>(Y, acc[m], pt, a, aa, M, lY, da, dpt);
+                        if constexpr (std::is_same<R, float>::value) {
+                            Vec6 vy, vl;
+#pragma unroll
+                            for (int c = 0; c < 6; ++c) {
+                                vy.v[c] = Y[c];
+                                vl.v[c] = acc[m][c];
+                            }
+                            const VjpOut o = rhs_vjp_call(vy, vl, pt, a, aa, M);
+#pragma unroll
+                            for (int c = 0; c < 6; ++c) lY[c] = o.y[c];
+                            da = o.da;
+                            dpt = o.dpt;
+                        } else {
+                            rhs_vjp<R>(Y, acc[m], pt, a, aa, M, lY, da, dpt);
+                        }
                         ga += da;
                         lpt += dpt;
 #pragma unroll
@@ -920,7 +956,7 @@ cudaError_t launch_diff_forward(const Scene& sc, const Camera& cam, const Camera
                                 cudaStream_t st, bool float_records) {
     const unsigned n = (unsigned)sc.width * (unsigned)sc.height;
     if (n == 0) return cudaSuccess;
-    const dim3 grid((n + 127) / 128);
+    const dim3 grid(unit_count(sc.width, sc.height, 1, false) / 4);  // 128 pixels of a 16x16 tile each
     if (sc.precision == 2 && float_records) {
         if (!replay) return cudaErrorInvalidValue;
         diff_forward_kernel<double, true, float><<<grid, 128, 0, st>>>(sc, cam, camd, rec, hdr, hdr64, err, flags);

@@ -76,6 +76,26 @@ struct Tally {
     }
 };
 
+// Unit index -> pixel in 16x16 tiles (raster order), Morton order inside a tile: an aligned run of
+// 32, 16, 8, ... indices is a patch of 8x4, 4x4, 4x2, ... pixels.  The index space covers whole
+// tiles, so at the right and bottom border it names pixels outside the frame.
+__device__ __forceinline__ void tile_to_pixel(unsigned idx, int W, int& px, int& py) {
+    const unsigned tiles_x = ((unsigned)W + 15u) >> 4;
+    const unsigned tile = idx >> 8, m = idx & 255u;
+    const unsigned ty = tile / tiles_x, tx = tile - ty * tiles_x;
+    const unsigned x = (m & 1u) | (m >> 1 & 2u) | (m >> 2 & 4u) | (m >> 3 & 8u);
+    const unsigned y = (m >> 1 & 1u) | (m >> 2 & 2u) | (m >> 3 & 4u) | (m >> 4 & 8u);
+    px = (int)(tx * 16u + x);
+    py = (int)(ty * 16u + y);
+}
+// Units of 32 / S pixels that cover a frame: whole tiles, or exactly its pixels when they come
+// from a pixel-order buffer.
+__host__ __device__ __forceinline__ unsigned unit_count(int W, int H, int S, bool ordered) {
+    const unsigned P = 32u / (unsigned)S;
+    const unsigned n = ordered ? (unsigned)W * (unsigned)H
+                               : ((unsigned)(W + 15) >> 4) * ((unsigned)(H + 15) >> 4) * 256u;
+    return (n + P - 1u) / P;
+}
 // Camera ray of sample `sample` of pixel (px, py) (cuda/kernel.cu:108-121): PCG jitter inside
 // the pixel, vertical field of view, aspect on u.  Stated-physics mode with one sample uses the
 // pixel centre.
