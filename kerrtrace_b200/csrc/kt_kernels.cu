@@ -96,18 +96,6 @@ __device__ __forceinline__ void unit_to_pixel(unsigned u, int W, int H, int& px,
     px = col0 + (int)(rem2 % (unsigned)wt);
 }
 
-// Lanes per pixel of the persistent tracer: the largest S <= min(spp, 32) that keeps 15 of 16
-// lanes busy over the pixel's samples (S lanes take spp samples in ceil(spp / S) rounds, and
-// 32 mod S lanes have no pixel).
-static int samples_in_parallel(int spp) {
-    int best = 1;
-    for (int S = 2; S <= 32 && S <= spp; ++S) {
-        const long long used = (long long)(32 / S) * spp, lanes = 32ll * ((spp + S - 1) / S);
-        if (16 * used >= 15 * lanes) best = S;
-    }
-    return best;
-}
-
 // ---- long-rays-first pixel order -----------------------------------------------------------
 // A ray that passes close to a spherical photon orbit winds around the hole about ln(1/delta)
 // times before it falls in or escapes, and takes several times the average step count.  Traced

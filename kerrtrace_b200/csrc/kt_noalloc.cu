@@ -7,15 +7,15 @@
 // in flight.  Such a caller cannot create a kt_context, which allocates its LUT textures and
 // its work counter.  kt_trace_noalloc takes everything from the caller instead — scene
 // configuration, cameras, the two LUTs as plain device arrays, the output buffers — and keeps
-// its only scratch, one work counter per view, in the file-scope array below.
+// its only scratch, a work counter, in the file-scope array below.
 //
 // The array is part of the library's device image: every GPU that loads the library holds its
 // 256 bytes until the process exits.  Every call shares it and it keeps the last call's
-// counters; each call clears the counters it uses on its own stream before the trace kernel
-// runs.  Calls that overlap on the GPU (other streams, other host threads on the same device)
-// race on the counters and must be serialised by the caller.
+// count; a call that uses it clears it on its own stream before the trace kernel runs.  Calls that
+// overlap on the GPU (other streams, other host threads on the same device) race on it and must
+// be serialised by the caller.
 //
-// The kernel is the persistent wavefront tracer with reference semantics; the LUTs are read
+// The kernel is the persistent tracer with reference semantics; the LUTs are read
 // from the plain arrays through a model of the texture unit's linear filter (mode 2 of the
 // device code), so results agree with kt_trace to the parity tolerance, not bit for bit.
 #include <cuda_runtime.h>
@@ -29,7 +29,7 @@
 
 namespace ktd {
 
-// Scratch of kt_trace_noalloc: one work counter per view.  In host code this name is only a
+// Scratch of kt_trace_noalloc: the work counter is its first word.  In host code this name is only a
 // stand-in for the device symbol; its device address comes from cudaGetSymbolAddress.
 static __device__ __align__(256) unsigned int g_noalloc_queue[KT_NOALLOC_MAX_VIEWS];
 
@@ -41,105 +41,59 @@ struct NoallocViews {
 constexpr unsigned kFullMask = 0xffffffffu;
 constexpr int kNoallocBlock = 128;
 
-// Same per-unit mapping as the wavefront kernel: 16-row bands, 16-column tiles, row-major.
-__device__ __forceinline__ void noalloc_unit_to_pixel(unsigned u, int W, int H, int& px, int& py) {
-    const unsigned band_px = (unsigned)W * 16u;
-    const unsigned band = u / band_px;
-    const unsigned rem = u - band * band_px;
-    const int row0 = (int)band * 16;
-    const int hb = min(16, H - row0);
-    const unsigned tile_px = 16u * (unsigned)hb;
-    const unsigned tile = rem / tile_px;
-    const unsigned rem2 = rem - tile * tile_px;
-    const int col0 = (int)tile * 16;
-    const int wt = min(16, W - col0);
-    py = row0 + (int)(rem2 / (unsigned)wt);
-    px = col0 + (int)(rem2 % (unsigned)wt);
-}
-
-// Persistent wavefront trace over several views of one scene.  A warp takes pixels from the
-// counter of its current view and moves to the next view when that counter is exhausted;
-// every lane remembers the view of the pixel it holds.
+// Persistent trace over several views of one scene, in the units of trace_wavefront_kernel: 32 / S
+// pixels with S samples of each side by side, view after view.  A warp's first unit is its own index
+// in the grid, the others come from one counter over all views.  (Refilling single lanes, as an
+// earlier form did, ran the ray set-up for one lane of 32: 8 views of 480x270 1.78 ms, now 1.26; at
+// 4 samples 8.55, now 4.59; 12 views of 64x36 at 2 samples 418 us, now 162.)
+template <bool TOGETHER>
 __global__ void __launch_bounds__(kNoallocBlock, 4)
     trace_views_noalloc_kernel(const __grid_constant__ Scene sc, const __grid_constant__ NoallocViews views,
-                               float4* __restrict__ hdr,
-                               uint32_t* __restrict__ err, unsigned* __restrict__ queue) {
+                               float4* __restrict__ hdr, uint32_t* __restrict__ err, unsigned* __restrict__ queue,
+                               int S) {
     constexpr int MODE = 2;
     const int lane = threadIdx.x & 31;
-    const unsigned lane_lt = (1u << lane) - 1u;
-    const unsigned n_units = (unsigned)sc.width * (unsigned)sc.height;
-    RayRun<float> ry;
-    Tally tl;
-    tl.clear();
-    int px = 0, py = 0, smp = 0, lview = 0, view = 0;
-    float acc[3] = {0.0f, 0.0f, 0.0f};
-    bool active = false;
-    bool open = views.n > 0;
-
-    while (true) {
-        if (open) {
-            const unsigned need = __ballot_sync(kFullMask, !active);
-            if (need) {
-                const int leader = __ffs(need) - 1;
-                const unsigned cnt = (unsigned)__popc(need);
-                unsigned base = 0;
-                if (lane == leader) base = atomicAdd(queue + view, cnt);
-                base = __shfl_sync(kFullMask, base, leader);
-                const int v = view;
-                if (base + cnt >= n_units) {
-                    ++view;
-                    if (view >= views.n) open = false;
-                }
-                if (!active) {
-                    const unsigned u = base + (unsigned)__popc(need & lane_lt);
-                    if (u < n_units) {
-                        lview = v;
-                        const Camera cam = views.cam[lview];
-                        noalloc_unit_to_pixel(u, sc.width, sc.height, px, py);
-                        acc[0] = acc[1] = acc[2] = 0.0f;
-                        for (smp = 0; smp < sc.spp; ++smp) {
-                            float dir[3];
-                            pixel_ray<MODE>(px, py, smp, sc, cam, dir);
-                            if (ray_start<float>(ry, cam, dir, sc)) break;
-                        }
-                        if (smp < sc.spp) {
-                            ray_prepare<float, MODE, false>(ry, sc, tl);
-                            active = true;
-                        } else {
-                            const float fs = sc.final_scale;
-                            hdr[(size_t)lview * n_units + (size_t)py * sc.width + px] =
-                                make_float4(acc[0] * fs, acc[1] * fs, acc[2] * fs, 1.0f);
-                        }
-                    }
-                }
-            }
-        }
-        // A warp with no ray in flight goes back for more pixels while views remain: a claim
-        // can come back empty (its view was used up, or every claimed pixel had no ray work,
-        // e.g. max_steps = 0), and `view` has then already moved on to the next view.
-        if (!__any_sync(kFullMask, active)) {
-            if (!open) break;
-            continue;
-        }
-        const int state = active ? ray_advance<float, MODE, false, false>(ry, sc, err + 2 * lview, tl, kRayGoing) : kRayGoing;
-        if (state != kRayGoing) {
-            acc[0] += ry.col[0];
-            acc[1] += ry.col[1];
-            acc[2] += ry.col[2];
-            const Camera cam = views.cam[lview];
-            for (++smp; smp < sc.spp; ++smp) {
+    const int slot = lane / S, sub = lane - slot * S;
+    const unsigned P = 32u / (unsigned)S;
+    const unsigned per_view = unit_count(sc.width, sc.height, S, false), units = per_view * (unsigned)views.n;
+    const unsigned n_warps = gridDim.x * (kNoallocBlock / 32);
+    const size_t n_px = (size_t)sc.width * sc.height;
+    for (unsigned u = blockIdx.x * (kNoallocBlock / 32) + (threadIdx.x >> 5); u < units;) {
+        const unsigned view = u / per_view;
+        const Camera& cam = views.cam[view];
+        int px, py;
+        tile_to_pixel((u - view * per_view) * P + (unsigned)slot, sc.width, px, py);
+        const bool valid = (unsigned)slot < P && px < sc.width && py < sc.height;
+        float acc[3] = {0.0f, 0.0f, 0.0f};
+        for (int s0 = 0; s0 < sc.spp; s0 += S) {
+            const int smp = s0 + sub;
+            RayRun<float> ry;
+            Tally tl;
+            bool run = false;
+            float col[3] = {0.0f, 0.0f, 0.0f};
+            if (valid && smp < sc.spp) {
                 float dir[3];
                 pixel_ray<MODE>(px, py, smp, sc, cam, dir);
-                if (ray_start<float>(ry, cam, dir, sc)) break;
+                run = ray_start<float>(ry, cam, dir, sc, smp > 0);
             }
-            if (smp < sc.spp) ray_prepare<float, MODE, false>(ry, sc, tl);
-            if (smp >= sc.spp) {
-                const float fs = sc.final_scale;
-                hdr[(size_t)lview * n_units + (size_t)py * sc.width + px] =
-                    make_float4(acc[0] * fs, acc[1] * fs, acc[2] * fs, 1.0f);
-                active = false;
+            run_rays<MODE, false, TOGETHER>(run, ry, sc, err + 2 * view, tl);
+            if (run) {
+#pragma unroll
+                for (int c = 0; c < 3; ++c) col[c] = ry.col[c];
+            }
+            const int last = min(S, sc.spp - s0);
+            for (int i = 0; i < last; ++i) {
+#pragma unroll
+                for (int c = 0; c < 3; ++c) acc[c] += __shfl_sync(kFullMask, col[c], min(slot * S + i, 31));
             }
         }
+        if (valid && sub == 0) {
+            const float fs = sc.final_scale;
+            hdr[view * n_px + (size_t)py * sc.width + px] = make_float4(acc[0] * fs, acc[1] * fs, acc[2] * fs, 1.0f);
+        }
+        if (units <= n_warps) break;
+        if (lane == 0) u = n_warps + atomicAdd(queue, 1u);
+        u = __shfl_sync(kFullMask, u, 0);
     }
 }
 
@@ -201,20 +155,29 @@ extern "C" kt_status kt_trace_noalloc(const kt_config* cfg, const kt_camera* cam
         }
         views.cam[v].fov_scale = cams[v].fov_scale;
     }
-    int dev = 0, sms = 0, per_sm = 0;
+    int dev = 0, sms = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return set_error(KT_ERR_CUDA, "cudaGetDevice failed");
     unsigned* queue = nullptr;
     if ((st = noalloc_scratch(dev, &queue)) != KT_OK) return st;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess ||
-        (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, trace_views_noalloc_kernel, kNoallocBlock, 0)) !=
-            cudaSuccess ||
-        (e = cudaMemsetAsync(queue, 0, n_views * sizeof(unsigned), s)) != cudaSuccess)
+    if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess)
         return set_error(KT_ERR_CUDA, cudaGetErrorString(e));
-    if (per_sm < 1) per_sm = 1;
-    trace_views_noalloc_kernel<<<sms * per_sm, kNoallocBlock, 0, s>>>(sc, views, reinterpret_cast<float4*>(hdr_out),
-                                                                     err_words, queue);
+    constexpr unsigned kWarps = kNoallocBlock / 32;
+    int S = samples_in_parallel(sc.spp);
+    // the unit counter is 32 bits wide (whole tiles of a large frame, up to a unit per pixel)
+    if ((uint64_t)unit_count(sc.width, sc.height, S, false) * n_views > 0x7fffffffu) S = 1;
+    const unsigned units = unit_count(sc.width, sc.height, S, false) * n_views;
+    const unsigned blocks = (units + kWarps - 1) / kWarps, resident = (unsigned)sms * 4u;
+    const unsigned grid = blocks < resident ? blocks : resident;
+    float4* hdr = reinterpret_cast<float4*>(hdr_out);
+    if (units <= grid * kWarps) {  // one unit per warp: lanes in step, as in launch_wave_minb
+        trace_views_noalloc_kernel<true><<<grid, kNoallocBlock, 0, s>>>(sc, views, hdr, err_words, queue, S);
+    } else {
+        if ((e = cudaMemsetAsync(queue, 0, sizeof(unsigned), s)) != cudaSuccess)
+            return set_error(KT_ERR_CUDA, cudaGetErrorString(e));
+        trace_views_noalloc_kernel<false><<<grid, kNoallocBlock, 0, s>>>(sc, views, hdr, err_words, queue, S);
+    }
     if ((e = cudaGetLastError()) != cudaSuccess) return set_error(KT_ERR_CUDA, cudaGetErrorString(e));
     return KT_OK;
 }

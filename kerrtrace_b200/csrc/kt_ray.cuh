@@ -96,6 +96,18 @@ __host__ __device__ __forceinline__ unsigned unit_count(int W, int H, int S, boo
                                : ((unsigned)(W + 15) >> 4) * ((unsigned)(H + 15) >> 4) * 256u;
     return (n + P - 1u) / P;
 }
+// Lanes per pixel of the persistent tracer: the largest S <= min(spp, 32) that keeps 15 of 16
+// lanes busy over the pixel's samples (S lanes take spp samples in ceil(spp / S) rounds, and
+// 32 mod S lanes have no pixel).
+inline int samples_in_parallel(int spp) {
+    int best = 1;
+    for (int S = 2; S <= 32 && S <= spp; ++S) {
+        const long long used = (long long)(32 / S) * spp, lanes = 32ll * ((spp + S - 1) / S);
+        if (16 * used >= 15 * lanes) best = S;
+    }
+    return best;
+}
+
 // Camera ray of sample `sample` of pixel (px, py) (cuda/kernel.cu:108-121): PCG jitter inside
 // the pixel, vertical field of view, aspect on u.  Stated-physics mode with one sample uses the
 // pixel centre.

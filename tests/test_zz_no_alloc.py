@@ -152,3 +152,16 @@ def test_noalloc_rejects_sizes_beyond_its_scratch(cuda):
     st = kt.lib().kt_trace_noalloc(C.byref(c), arr, 1, C.c_void_p(dummy.data_ptr()), C.c_void_p(dummy.data_ptr()),
                                    None, C.c_void_p(dummy.data_ptr()), C.c_void_p(dummy.data_ptr()))
     assert st == kt.KT_ERR_UNSUPPORTED
+
+
+@pytest.mark.parametrize("n_views,size,spp", [(5, (17, 9), 3), (3, (301, 203), 5), (1, (1, 1), 1)])
+def test_noalloc_ragged_views(cuda, n_views, size, spp):
+    """Views that are not whole 16x16 tiles, with several samples of a pixel side by side: fewer
+    units than warps and more."""
+    cfg, cam = workloads.scene("t1")
+    cfg = workloads.scaled(cfg, *size)
+    cfg.spp = spp
+    bb, disk = _luts(cuda, cfg)
+    cams = _views(cam, n_views)
+    hdr, err, _ = _noalloc(cuda, cfg, cams, bb, disk)
+    _check_views(cuda, cfg, cams, hdr, err)
