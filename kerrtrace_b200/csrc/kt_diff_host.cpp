@@ -8,6 +8,7 @@
 // Page-Thorne flux differentiated with dual numbers in double.  The FP64 path also takes theta,
 // the camera and the disk LUT in double, so that its image is a smooth function of theta down
 // to double rounding (which central differences of small steps need).
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -64,22 +65,35 @@ HD isco_d(HD an) {
     return HD(3.0) + z2 - hsqrt(inside);
 }
 
-// Page-Thorne flux factor (nt_factor_f32 of the host builders) in double with derivatives.
-HD nt_factor_d(HD r, HD an, HD r_isco, double inv_m) {
-    if (!(r.v > r_isco.v)) return HD(0.0);
-    const HD rn = r * HD(inv_m), rin = r_isco * HD(inv_m);
-    const HD x = hsqrt(rn), xms = hsqrt(rin);
+// Page-Thorne flux factor (nt_factor_f32 of the host builders) in double with derivatives.  What
+// depends on the spin and the ISCO alone is computed once per table (a forward call builds one).
+struct NtTermsD {
+    HD roots[3], den[3], coef[3], xms;
+};
+NtTermsD nt_terms_d(HD an, HD r_isco, double inv_m) {
+    NtTermsD t;
+    t.xms = hsqrt(r_isco * HD(inv_m));
     const HD base = hacos(-an) * HD(1.0 / 3.0);
     const double step = 2.0943951023931957;
-    const HD roots[3] = {HD(2.0) * hcos(base), HD(2.0) * hcos(base - HD(step)), HD(2.0) * hcos(base + HD(step))};
+    t.roots[0] = HD(2.0) * hcos(base);
+    t.roots[1] = HD(2.0) * hcos(base - HD(step));
+    t.roots[2] = HD(2.0) * hcos(base + HD(step));
+    for (int i = 0; i < 3; ++i) {
+        const HD xi = t.roots[i];
+        t.den[i] = xi * (xi - t.roots[(i + 1) % 3]) * (xi - t.roots[(i + 2) % 3]);
+        t.coef[i] = HD(3.0) * (xi - an) * (xi - an) / t.den[i];
+    }
+    return t;
+}
+HD nt_factor_d(HD r, HD an, HD r_isco, double inv_m, const NtTermsD& t) {
+    if (!(r.v > r_isco.v)) return HD(0.0);
+    const HD rn = r * HD(inv_m);
+    const HD x = hsqrt(rn), xms = t.xms;
     HD sum(0.0);
     for (int i = 0; i < 3; ++i) {
-        const HD xi = roots[i];
-        const HD den = xi * (xi - roots[(i + 1) % 3]) * (xi - roots[(i + 2) % 3]);
-        if (!(den.v > 0.0)) continue;
-        const HD coef = HD(3.0) * (xi - an) * (xi - an) / den;
-        const HD val = (x - xi) / (xms - xi);
-        if (val.v > 0.0) sum = sum + coef * hlog(val);
+        if (!(t.den[i].v > 0.0)) continue;
+        const HD val = (x - t.roots[i]) / (xms - t.roots[i]);
+        if (val.v > 0.0) sum = sum + t.coef[i] * hlog(val);
     }
     const HD q = x - xms - HD(1.5) * an * hlog(x / xms) - sum;
     const HD geo = rn * (rn * x - HD(3.0) * x + HD(2.0) * an);
@@ -156,12 +170,13 @@ ktd::Camera to_dev_camera(const kt_camera& c) {
 
 }  // namespace
 
-// One LUT set per parameter point in use (the recorded one, and the replay one).
+// One LUT set per parameter point in use (the recorded one, and the replay one), in one block of
+// device memory that one copy fills.
 struct kt_diff_luts {
-    float* disk = nullptr;       // float LUT (FP32 path: the renderer's LUT)
-    double* disk_d = nullptr;    // double LUT (FP64 path)
+    double* disk_d = nullptr;    // double LUT (FP64 path); the block's start
     double* dlut_da = nullptr;
     double* dlut_dro = nullptr;
+    float* disk = nullptr;       // float LUT (FP32 path: the renderer's LUT)
 };
 
 struct kt_diff {
@@ -188,10 +203,7 @@ struct kt_diff {
 namespace {
 
 void free_luts(kt_diff_luts& l) {
-    cudaFree(l.disk);
     cudaFree(l.disk_d);
-    cudaFree(l.dlut_da);
-    cudaFree(l.dlut_dro);
     l = kt_diff_luts{};
 }
 
@@ -228,19 +240,21 @@ kt_status prepare(kt_diff* d, const kt_diff_params* th, kt_diff_luts& luts, cuda
     kt_kerr_params kp;
     if ((s = kt_build_kerr_params(&c, &kp)) != KT_OK) return s;
     const uint32_t n = c.lut_size;
-    std::vector<float> disk(n);
-    std::vector<double> disk_d(n), da(n), dro(n);
-    if ((s = kt_generate_disk_lut(&kp, c.disk_outer_radius, n, disk.data())) != KT_OK) return s;
+    // the tables in the order of the device block: three double ones, the float one
+    std::vector<double> block(3 * (size_t)n + (n + 1) / 2);
+    double *disk_d = block.data(), *da = disk_d + n, *dro = da + n;
+    if ((s = kt_generate_disk_lut(&kp, c.disk_outer_radius, n, reinterpret_cast<float*>(dro + n))) != KT_OK) return s;
     // entries f(r_i)^(1/4), r_i = r_in + i / (n - 1) (r_out - r_in), with their derivatives
     const double m = (double)c.mass, inv_m = 1.0 / m;
     const HD an(th->spin * inv_m, inv_m, 0.0);
     const HD r_in = isco_d(an) * HD(m);
     const HD r_out(th->disk_outer_radius, 0.0, 1.0);
     if (!(r_out.v > r_in.v)) return err_arg("disk outer radius must exceed the ISCO");
+    const NtTermsD terms = nt_terms_d(an, r_in, inv_m);
     for (uint32_t i = 0; i < n; ++i) {
         const double ratio = (double)i / (double)(n - 1);
         const HD r = r_in + HD(ratio) * (r_out - r_in);
-        const HD f = nt_factor_d(r, an, r_in, inv_m);
+        const HD f = nt_factor_d(r, an, r_in, inv_m, terms);
         double v = 0.0, g0 = 0.0, g1 = 0.0;
         if (f.v > 0.0) {
             v = std::pow(f.v, 0.25);
@@ -252,13 +266,15 @@ kt_status prepare(kt_diff* d, const kt_diff_params* th, kt_diff_luts& luts, cuda
         da[i] = g0;
         dro[i] = g1;
     }
-    cudaError_t e;
-    if ((e = cudaMemcpyAsync(luts.disk, disk.data(), n * sizeof(float), cudaMemcpyHostToDevice, st)) != cudaSuccess ||
-        (e = cudaMemcpyAsync(luts.disk_d, disk_d.data(), n * sizeof(double), cudaMemcpyHostToDevice, st)) != cudaSuccess ||
-        (e = cudaMemcpyAsync(luts.dlut_da, da.data(), n * sizeof(double), cudaMemcpyHostToDevice, st)) != cudaSuccess ||
-        (e = cudaMemcpyAsync(luts.dlut_dro, dro.data(), n * sizeof(double), cudaMemcpyHostToDevice, st)) != cudaSuccess)
-        return err_cuda(e, "diff LUT upload");
-    // pageable sources: the copies have been staged when cudaMemcpyAsync returns
+    // pageable source: a copy has been staged when cudaMemcpyAsync returns, without waiting for the
+    // stream up to 64 KB (one copy at 1024 entries)
+    const size_t total = n * (3 * sizeof(double) + sizeof(float)), piece = 48 * 1024;
+    for (size_t at = 0; at < total; at += piece) {
+        const cudaError_t e = cudaMemcpyAsync(reinterpret_cast<char*>(luts.disk_d) + at,
+                                              reinterpret_cast<const char*>(block.data()) + at,
+                                              std::min(piece, total - at), cudaMemcpyHostToDevice, st);
+        if (e != cudaSuccess) return err_cuda(e, "diff LUT upload");
+    }
     sc->bb_lut = d->bb;
     sc->disk_lut = luts.disk;
     sc->bb_tex = 0;
@@ -348,13 +364,13 @@ kt_status kt_diff_create(const kt_config* cfg, const kt_diff_view* view, uint32_
         return err_cuda(e, "diff allocation");
     }
     for (kt_diff_luts* l : {&d->lut_rec, &d->lut_rep}) {
-        if ((e = cudaMalloc(&l->disk, n * sizeof(float))) != cudaSuccess ||
-            (e = cudaMalloc(&l->disk_d, n * sizeof(double))) != cudaSuccess ||
-            (e = cudaMalloc(&l->dlut_da, n * sizeof(double))) != cudaSuccess ||
-            (e = cudaMalloc(&l->dlut_dro, n * sizeof(double))) != cudaSuccess) {
+        if ((e = cudaMalloc(&l->disk_d, n * (3 * sizeof(double) + sizeof(float)))) != cudaSuccess) {
             destroy(d);
             return err_cuda(e, "diff LUT allocation");
         }
+        l->dlut_da = l->disk_d + n;
+        l->dlut_dro = l->dlut_da + n;
+        l->disk = reinterpret_cast<float*>(l->dlut_dro + n);
     }
     *out = d;
     return KT_OK;

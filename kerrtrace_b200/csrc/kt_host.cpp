@@ -57,10 +57,21 @@ kt_status cuda_fail(cudaError_t e, const char* what) {
 // ---- numeric helpers ---------------------------------------------------------------------
 
 // src/math.rs:15-32: the f64 is printed with its shortest round-trip digits and that text is
-// parsed as f32.
+// parsed as f32.  The text's value lies within half an ulp of the f64, so it rounds to the same f32
+// as the f64 itself unless the midpoint of two f32 is that close: only then (and for subnormal
+// results) the text is made (about 150 ns against 2; the tables convert every entry).
 bool f32_from_f64(double v, float* out) {
     if (!std::isfinite(v)) return false;
     if (v < -(double)std::numeric_limits<float>::max() || v > (double)std::numeric_limits<float>::max()) return false;
+    uint64_t bits;
+    std::memcpy(&bits, &v, sizeof bits);
+    const uint32_t below = (uint32_t)(bits & 0x1fffffffu);  // the 29 bits that f32 does not keep
+    if ((below < 0x0fffffffu || below > 0x10000001u) && std::fabs(v) >= (double)std::numeric_limits<float>::min()) {
+        const float f = (float)v;
+        if (!std::isfinite(f)) return false;
+        *out = f;
+        return true;
+    }
     char buf[64];
     auto res = std::to_chars(buf, buf + sizeof buf - 1, v);
     if (res.ec != std::errc()) return false;
@@ -97,26 +108,37 @@ float isco_f32(float a_norm, bool prograde, float mass) {
     return mass * (3.0f + z2 + sign * sqrtf(fmaxf(inside, 0.0f)));
 }
 
-// Page-Thorne flux factor with the roots 2 cos(acos(-a)/3 - 2 pi k / 3) of x^3 - 3x + 2a = 0.
-float nt_factor_f32(float r, float a_norm, float r_isco, float inv_m) {
-    if (r <= r_isco) return 0.0f;
-    const float r_norm = r * inv_m;
-    const float r_isco_norm = r_isco * inv_m;
-    const float x = sqrtf(r_norm);
-    const float x_ms = sqrtf(r_isco_norm);
+// Page-Thorne flux factor with the roots 2 cos(acos(-a)/3 - 2 pi k / 3) of x^3 - 3x + 2a = 0.  What
+// depends on the spin and the ISCO alone is computed once per table.
+struct NtTerms {
+    float roots[3], den[3], coef[3], x_ms;
+};
+NtTerms nt_terms_f32(float a_norm, float r_isco, float inv_m) {
+    NtTerms t;
+    t.x_ms = sqrtf(r_isco * inv_m);
     const float third = 1.0f / 3.0f;
     const float angle_base = acosf(-a_norm) * third;
     const float ang_step = 2.0943952f;
-    const float roots[3] = {2.0f * cosf(angle_base), 2.0f * cosf(angle_base - ang_step),
-                            2.0f * cosf(angle_base + ang_step)};
+    t.roots[0] = 2.0f * cosf(angle_base);
+    t.roots[1] = 2.0f * cosf(angle_base - ang_step);
+    t.roots[2] = 2.0f * cosf(angle_base + ang_step);
+    for (int i = 0; i < 3; ++i) {
+        const float xi = t.roots[i];
+        t.den[i] = xi * (xi - t.roots[(i + 1) % 3]) * (xi - t.roots[(i + 2) % 3]);
+        t.coef[i] = 3.0f * (xi - a_norm) * (xi - a_norm) / t.den[i];
+    }
+    return t;
+}
+float nt_factor_f32(float r, float a_norm, float r_isco, float inv_m, const NtTerms& t) {
+    if (r <= r_isco) return 0.0f;
+    const float r_norm = r * inv_m;
+    const float x = sqrtf(r_norm);
+    const float x_ms = t.x_ms;
     float sum_log = 0.0f;
     for (int i = 0; i < 3; ++i) {
-        const float xi = roots[i];
-        const float den = xi * (xi - roots[(i + 1) % 3]) * (xi - roots[(i + 2) % 3]);
-        if (den <= 0.0f) continue;
-        const float coef = 3.0f * (xi - a_norm) * (xi - a_norm) / den;
-        const float val = (x - xi) / (x_ms - xi);
-        if (val > 0.0f) sum_log += coef * logf(val);
+        if (t.den[i] <= 0.0f) continue;
+        const float val = (x - t.roots[i]) / (x_ms - t.roots[i]);
+        if (val > 0.0f) sum_log += t.coef[i] * logf(val);
     }
     const float q = fmaf(1.5f * a_norm, -logf(x / x_ms), x - x_ms) - sum_log;
     const float geo = r_norm * fmaf(2.0f, a_norm, fmaf(r_norm, x, -(3.0f * x)));
@@ -256,9 +278,11 @@ kt_status kt_generate_blackbody_lut(uint32_t size, float max_temp, float wl_star
         if (lambdas.size() > (1u << 24)) return fail(KT_ERR_INVALID_ARG, "wavelength grid too large");
     }
     const size_t n = lambdas.size();
-    std::vector<float> xs(n), ys(n), zs(n);
+    std::vector<float> xs(n), ys(n), zs(n), inv_l5(n);
     for (size_t i = 0; i < n; ++i) {
         const float l = lambdas[i];
+        const float l2 = l * l;
+        inv_l5[i] = 1.0f / (l * (l2 * l2));
         xs[i] = cmf_lobe(l, 1.056f, 599.8f, 37.9f, 31.0f) + cmf_lobe(l, 0.362f, 442.0f, 16.0f, 26.7f) +
                 cmf_lobe(l, -0.065f, 501.1f, 20.4f, 26.2f);
         ys[i] = cmf_lobe(l, 0.821f, 568.8f, 46.9f, 40.5f) + cmf_lobe(l, 0.286f, 530.9f, 16.3f, 31.1f);
@@ -278,11 +302,7 @@ kt_status kt_generate_blackbody_lut(uint32_t size, float max_temp, float wl_star
             if (t > 0.0f) {
                 const float l = lambdas[i];
                 const float expo = c2 / (l * t);
-                if (!(expo > 80.0f)) {
-                    const float l2 = l * l;
-                    const float l5 = l * (l2 * l2);
-                    inten = ((1.0f / l5) / expm1f(expo)) * 1e15f;
-                }
+                if (!(expo > 80.0f)) inten = (inv_l5[i] / expm1f(expo)) * 1e15f;
             }
             xsum += inten * xs[i];
             ysum += inten * ys[i];
@@ -337,11 +357,12 @@ kt_status kt_generate_disk_lut(const kt_kerr_params* p, float disk_outer, uint32
                     disk_outer, p->disk_inner);
     const double inner = (double)p->disk_inner;
     const double span = (double)(disk_outer - p->disk_inner);
+    const NtTerms terms = nt_terms_f32(p->a_norm, p->disk_inner, p->inv_m);
     for (uint32_t i = 0; i < size; ++i) {
         const double ratio = (double)i / (double)(size - 1);
         float r;
         if (!f32_from_f64(std::fma(ratio, span, inner), &r)) return fail(KT_ERR_INVALID_ARG, "disk radius conversion failed");
-        const float f = nt_factor_f32(r, p->a_norm, p->disk_inner, p->inv_m);
+        const float f = nt_factor_f32(r, p->a_norm, p->disk_inner, p->inv_m, terms);
         if (!std::isfinite(f)) return fail(KT_ERR_INVALID_ARG, "disk flux factor is not finite");
         const float v = sqrtf(sqrtf(f));
         if (!std::isfinite(v)) return fail(KT_ERR_INVALID_ARG, "disk temperature factor is not finite");

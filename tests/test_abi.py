@@ -294,3 +294,16 @@ def test_autotune_through_the_c_abi(kt):
     assert kt.lib().kt_context_autotune(ctx.handle, None, C.byref(cam), 1, C.byref(bad), 0, None, None) == \
         kt.KT_ERR_INVALID_ARG
     ctx.close()
+
+
+@pytest.mark.parametrize("spin,mass,span,size", [(0.0, 1.0, 5.0, 2), (0.5, 1.0, 1e-3, 333), (-0.9, 1.0, 40.0, 1024),
+                                                 (0.998, 1.0, 24.0, 4096), (-0.45, 0.5, 37.7, 1000), (2.1, 2.3, 60.0, 64)])
+def test_disk_tables_equal_the_oracle_restatement(kt, orc, spin, mass, span, size):
+    """Tables whose spin terms are computed once and whose radii skip the decimal text where it cannot
+    matter: bit for bit the oracle's, which computes every entry in full."""
+    cfg = kt.config_default()
+    cfg.spin, cfg.mass = spin, mass
+    p = kt.build_kerr_params(cfg)
+    r_out = float(np.float32(p.disk_inner + span))
+    got = kt.generate_disk_lut(p, r_out, size)
+    assert np.array_equal(got.view(np.uint32), orc.disk_lut(cfg.spin, cfg.mass, r_out, size).view(np.uint32))
