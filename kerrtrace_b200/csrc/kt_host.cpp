@@ -1226,7 +1226,7 @@ void batch_layout(kt_batch* b) {
         e.tile_begin = tiles;
         tiles += e.tiles_x * tiles_y;
         e.unit_begin = units;
-        units += (unsigned)(((uint64_t)e.sc.width * e.sc.height + 31) / 32);
+        units += ktd::unit_count(e.sc.width, e.sc.height, 1, false);
     }
     b->table->total_tiles = tiles;
     b->table->total_units = units;

@@ -48,6 +48,15 @@ cudaError_t launch_trace(const Scene& sc, const Camera& cam, int schedule, float
                          uint32_t* err, unsigned* queue, unsigned long long* ctr, float4* aux,
                          const Tuning& tn, int bx, int by, unsigned* order, cudaStream_t stream);
 
+// Units of 32 / S pixels that cover a frame: whole tiles, or exactly its pixels when they come
+// from a pixel-order buffer.
+__host__ __device__ inline unsigned unit_count(int W, int H, int S, bool ordered) {
+    const unsigned P = 32u / (unsigned)S;
+    const unsigned n = ordered ? (unsigned)W * (unsigned)H
+                               : ((unsigned)(W + 15) >> 4) * ((unsigned)(H + 15) >> 4) * 256u;
+    return (n + P - 1u) / P;
+}
+
 // Batched trace: one plain-schedule launch over the tiles of up to kBatchMaxJobs renders.  The
 // table travels as a kernel parameter (__grid_constant__); each block finds its job from the
 // tile prefix, so the job index and its scene constants are uniform across the block.

@@ -467,21 +467,24 @@ cudaError_t launch_batch(const BatchTable& bt, int bx, int by, cudaStream_t st) 
     return launch_batch_typed<float, 0>(bt, bx, by, st);
 }
 
-// Persistent batched trace.  The pixels of every job are cut into units of 32 (the tile order of
-// unit_to_pixel, so a unit is a 16x2 patch of one frame); job j owns units [unit_begin,
-// unit_begin of j + 1).  A warp takes one unit at a time from a single device counter over all
-// jobs, so the 32 rays of a warp always share one scene and its parameters stay uniform
+// Persistent batched trace.  Every job is cut into units of 32 pixels (tile_to_pixel's order, so a
+// unit is an 8x4 patch of one frame); job j owns units [unit_begin, unit_begin of j + 1).  A
+// warp's first unit is its own index in the grid, the others come from a single device counter
+// over all jobs, so the 32 rays of a warp always share one scene and its parameters stay uniform
 // constant-bank loads, and an SM never waits for a whole block: each warp moves on as soon as
 // its own unit is done.  Per-pixel arithmetic is the plain kernel's (run_ray).
-template <class R, int MODE, int MINB>
+//
+// Bound by the FP32 pipe; lanes idle while the longest ray of their unit finishes, and a square
+// patch holds rays more alike than one of 16x2: 64 renders of 128x128 to 960x540 15.75 -> 15.45
+// ms, 64 up to 400x225 3.01 -> 2.95.  A batch of one unit per warp at most lasts as long as its
+// longest ray, and takes the loop that keeps a warp's lanes in step (TOGETHER): two renders of
+// 100 columns 130 -> 104 us, five of up to 160 181 -> 130.
+template <class R, int MODE, int MINB, bool TOGETHER>
 __global__ void __launch_bounds__(kWavefrontBlock, MINB)
     trace_batch_persistent_kernel(const __grid_constant__ BatchTable bt, unsigned* __restrict__ counter) {
     const int lane = threadIdx.x & 31;
-    while (true) {
-        unsigned u = 0;
-        if (lane == 0) u = atomicAdd(counter, 1u);
-        u = __shfl_sync(kFull, u, 0);
-        if (u >= bt.total_units) break;
+    const unsigned n_warps = gridDim.x * (kWavefrontBlock / 32);
+    for (unsigned u = blockIdx.x * (kWavefrontBlock / 32) + (threadIdx.x >> 5); u < bt.total_units;) {
         int lo = 0, hi = bt.n - 1;  // last job whose first unit is <= u
         while (lo < hi) {
             const int mid = (lo + hi + 1) >> 1;
@@ -489,19 +492,21 @@ __global__ void __launch_bounds__(kWavefrontBlock, MINB)
         }
         const BatchJob& jb = bt.job[lo];
         const Scene& sc = jb.sc;
-        const unsigned pix = (u - jb.unit_begin) * 32u + (unsigned)lane;
-        const bool valid = pix < (unsigned)sc.width * (unsigned)sc.height;
-        int px = 0, py = 0;
-        if (valid) unit_to_pixel(pix, sc.width, sc.height, px, py);
+        int px, py;
+        tile_to_pixel((u - jb.unit_begin) * 32u + (unsigned)lane, sc.width, px, py);
+        const bool valid = px < sc.width && py < sc.height;
         float acc[3] = {0.0f, 0.0f, 0.0f};
         Tally total;
         total.clear();
         for (int smp = 0; smp < sc.spp; ++smp)
-            run_ray<R, MODE, false, false>(valid, px, py, smp, sc, jb.cam, jb.err, acc, total, nullptr);
+            run_ray<R, MODE, false, TOGETHER>(valid, px, py, smp, sc, jb.cam, jb.err, acc, total, nullptr);
         if (valid) {
             const float fs = sc.final_scale;
             jb.hdr[py * sc.width + px] = make_float4(acc[0] * fs, acc[1] * fs, acc[2] * fs, 1.0f);
         }
+        if (bt.total_units <= n_warps) break;
+        if (lane == 0) u = n_warps + atomicAdd(counter, 1u);
+        u = __shfl_sync(kFull, u, 0);
     }
 }
 
@@ -511,12 +516,18 @@ static cudaError_t launch_batch_persistent_minb(const BatchTable& bt, unsigned* 
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
     if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
-    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, trace_batch_persistent_kernel<R, MODE, MINB>,
+    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, trace_batch_persistent_kernel<R, MODE, MINB, false>,
                                                            kWavefrontBlock, 0)) != cudaSuccess)
         return e;
     if (per_sm < 1) per_sm = 1;
+    const unsigned warps = (unsigned)(sms * per_sm) * (kWavefrontBlock / 32);
+    if (bt.total_units <= warps) {
+        const unsigned blocks = (bt.total_units + kWavefrontBlock / 32 - 1) / (kWavefrontBlock / 32);
+        trace_batch_persistent_kernel<R, MODE, MINB, true><<<blocks, kWavefrontBlock, 0, st>>>(bt, counter);
+        return cudaGetLastError();
+    }
     if ((e = cudaMemsetAsync(counter, 0, sizeof(unsigned), st)) != cudaSuccess) return e;
-    trace_batch_persistent_kernel<R, MODE, MINB><<<sms * per_sm, kWavefrontBlock, 0, st>>>(bt, counter);
+    trace_batch_persistent_kernel<R, MODE, MINB, false><<<sms * per_sm, kWavefrontBlock, 0, st>>>(bt, counter);
     return cudaGetLastError();
 }
 

@@ -88,14 +88,6 @@ __device__ __forceinline__ void tile_to_pixel(unsigned idx, int W, int& px, int&
     px = (int)(tx * 16u + x);
     py = (int)(ty * 16u + y);
 }
-// Units of 32 / S pixels that cover a frame: whole tiles, or exactly its pixels when they come
-// from a pixel-order buffer.
-__host__ __device__ __forceinline__ unsigned unit_count(int W, int H, int S, bool ordered) {
-    const unsigned P = 32u / (unsigned)S;
-    const unsigned n = ordered ? (unsigned)W * (unsigned)H
-                               : ((unsigned)(W + 15) >> 4) * ((unsigned)(H + 15) >> 4) * 256u;
-    return (n + P - 1u) / P;
-}
 // Lanes per pixel of the persistent tracer: the largest S <= min(spp, 32) that keeps 15 of 16
 // lanes busy over the pixel's samples (S lanes take spp samples in ceil(spp / S) rounds, and
 // 32 mod S lanes have no pixel).

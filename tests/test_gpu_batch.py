@@ -162,3 +162,27 @@ def test_persistent_batch_of_64_ragged_jobs(cuda):
             assert np.all(got[:, 3] == 1.0)
             assert np.array_equal(got.view(np.uint32), exp.view(np.uint32))
     b.close()
+
+
+@pytest.mark.parametrize("mode,prec", [(kt.MODE_REF, kt.PREC_FP32), (kt.MODE_SPEC, kt.PREC_FP32),
+                                       (kt.MODE_SPEC, kt.PREC_MIXED), (kt.MODE_SPEC, kt.PREC_FP64)])
+@pytest.mark.parametrize("sizes", [[(17, 33), (1, 5), (48, 16)], [(401, 303), (15, 1), (333, 47)]])
+def test_persistent_batch_units(cuda, mode, prec, sizes):
+    """Persistent batches of one unit per resident warp at most, and of more units than that, in
+    frames whose last tiles are cut in both directions: equal to each job's own plain trace."""
+    base, cam = workloads.scene("t1")
+    jobs = []
+    for w, h in sizes:
+        c = workloads.scaled(base, w, h)
+        c.mode, c.precision, c.max_steps = mode, prec, 150
+        c.disk_temperature_scale = base.disk_temperature_scale
+        jobs.append((c, cam))
+    bufs = _alloc(cuda, jobs)
+    b = kt.Batch([(c, cam, h.data_ptr(), e.data_ptr()) for (c, cam), (h, e) in zip(jobs, bufs)])
+    b.set_tuning(kt.SCHED_WAVEFRONT, blocks_per_sm=5)
+    b.trace()
+    cuda.cuda.synchronize()
+    for (c, cam), (h, _) in zip(jobs, bufs):
+        exp = run_ours(cuda, c, cam, kt.SCHED_PLAIN)[0]
+        assert np.array_equal(h.cpu().numpy().view(np.uint32), exp.view(np.uint32)), (c.width, c.height)
+    b.close()
