@@ -257,6 +257,7 @@ __global__ void __launch_bounds__(kWavefrontBlock, MINB)
                            uint32_t* __restrict__ err, unsigned* __restrict__ queue,
                            unsigned long long* __restrict__ ctr, float4* __restrict__ aux, int S,
                            const unsigned* __restrict__ order) {
+    if (TOGETHER) wait_for_stream();
     const int lane = threadIdx.x & 31;
     const int slot = lane / S, sub = lane - slot * S;
     const unsigned P = 32u / (unsigned)S;
@@ -373,9 +374,13 @@ static cudaError_t launch_wave_minb(const Scene& sc, const Camera& cam, float4* 
     // moves around it cost more than they save (1920x1080 2.21 -> 2.37 ms).
     if constexpr (!COUNT && MINB == WaveDefaults<R>::minb) {
         if (units <= resident * kWarps) {
-            trace_wavefront_kernel<R, MODE, COUNT, MINB, true>
-                <<<grid, kWavefrontBlock, 0, st>>>(sc, cam, hdr, err, queue, ctr, aux, S, order);
-            return cudaGetLastError();
+            if (order) {
+                trace_wavefront_kernel<R, MODE, COUNT, MINB, true>
+                    <<<grid, kWavefrontBlock, 0, st>>>(sc, cam, hdr, err, queue, ctr, aux, S, order);
+                return cudaGetLastError();
+            }
+            return launch_early(trace_wavefront_kernel<R, MODE, COUNT, MINB, true>, dim3(grid), kWavefrontBlock, 0, st, sc,
+                                cam, hdr, err, queue, ctr, aux, S, order);
         }
     }
     trace_wavefront_kernel<R, MODE, COUNT, MINB, false>
@@ -625,10 +630,11 @@ __device__ __forceinline__ float4 bloom_source(float4 c, const PostParams& pp) {
 // plain multiply-adds of an earlier form competed with them for slots and kept the pipe 37% busy.
 // 64 x 32-pixel tiles of 128 threads: 43 KB and 5 blocks per SM at R = 24, 7 blocks per SM and
 // frame at 1920x1080 (1020 blocks: a 128-wide tile would leave some SMs 4 and some 3).  Both passes
-// back to back (fused): 1920x1080 R = 24 66.4 -> 45.3 us, 3840x2160 213 -> 168 us, 2100x900 R = 48 118
-// -> 68.9 us, 960x540 30.9 -> 21.0 us.  Without the blur 1920x1080 takes 31 us and without the staging 41:
-// what is left beside the multiply-adds (18 us) is each block's chain of loads, tone map and
-// stores with 16 to 20 warps per SM to cover it.
+// back to back (fused), their launches overlapped (launch_early): 1920x1080 R = 24 66.4 -> 40.8 us,
+// 3840x2160 213 -> 159 us, 2100x900 R = 48 118 -> 64.4 us, 960x540 30.9 -> 16.2 us.  Without the
+// overlap 1920x1080 takes 45.3 us, without the blur as well 31, without the staging 41: what is left
+// beside the multiply-adds (18 us) is each block's chain of loads, tone map and stores with 16 to
+// 20 warps per SM to cover it.
 constexpr int kBJ = 8, kTPairs = 16, kTPos = 64, kTThreads = kTPairs * (kTPos / kBJ);
 constexpr int kTWarps = kTThreads / 32;
 
@@ -748,8 +754,8 @@ __device__ __forceinline__ void load_row_pair(const float4* row, int W, float4 (
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
         if (32 * q < left) {
-            u[q] = __ldg(row + 32 * q);
-            v[q] = __ldg(row + W + 32 * q);
+            u[q] = load_behind_wait(row + 32 * q);
+            v[q] = load_behind_wait(row + W + 32 * q);
         }
     }
 }
@@ -807,7 +813,9 @@ __global__ void __launch_bounds__(kTThreads, 5) bloom_h_kernel(const PostParams 
     const PairTile t = pair_tile(smem_raw, R);
     const int x0 = blockIdx.x * kTPos, y0 = blockIdx.y * (2 * kTPairs);
     const int tid = threadIdx.x;
+    if (PAIRED) let_next_launch();
     stage_tables(t, pp, pp.inv_wsum_x, x0, W, tid);
+    wait_for_stream();
     {
         // a warp takes 4 row pairs, 128 columns of one at a time: 8 loads in flight per lane
         const int warp = tid >> 5, lane = tid & 31;
@@ -835,8 +843,8 @@ __global__ void __launch_bounds__(kTThreads, 5) bloom_h_kernel(const PostParams 
                     for (int q = 0; q < 4; ++q) {
                         const int c = c0 + 32 * q, x = x0 - R + lane + c;
                         const bool in = x >= 0 && x < W && lane + c < segw;
-                        u[q] = in && y < H ? __ldg(src + c) : make_float4(0.f, 0.f, 0.f, 0.f);
-                        v[q] = in && y + 1 < H ? __ldg(src + W + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+                        u[q] = in && y < H ? load_behind_wait(src + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+                        v[q] = in && y + 1 < H ? load_behind_wait(src + W + c) : make_float4(0.f, 0.f, 0.f, 0.f);
                     }
                     store_row_pair(u, v, rg + c0, b + c0, segw - c0 - lane, pp);
                 }
@@ -910,6 +918,7 @@ __global__ void __launch_bounds__(kTThreads, 4) post_v_kernel(const PostParams p
     const int x0 = blockIdx.x * (2 * kTPairs), y0 = blockIdx.y * kTPos;
     const int tid = threadIdx.x;
     stage_tables(t, pp, pp.inv_wsum_y, y0, H, tid);
+    wait_for_stream();
     if (PAIRED) {
         const int warp = tid >> 5, lane = tid & 31;
         const size_t pairs = bloom_pairs(W);
@@ -946,8 +955,8 @@ __global__ void __launch_bounds__(kTThreads, 4) post_v_kernel(const PostParams p
             const bool in = y >= 0 && y < H;
             const float4* row = bloom + (size_t)(in ? y : 0) * W;
             float4 u = make_float4(0.f, 0.f, 0.f, 0.f), v = u;
-            if (in && x < W) u = __ldg(row + x);
-            if (in && x + 1 < W) v = __ldg(row + x + 1);
+            if (in && x < W) u = load_behind_wait(row + x);
+            if (in && x + 1 < W) v = load_behind_wait(row + x + 1);
             t.rg[p * stride + c] = make_ulonglong2(pack2(u.x, v.x), pack2(u.y, v.y));
             t.b[p * stride + c] = pack2(u.z, v.z);
         }
@@ -967,8 +976,8 @@ __global__ void __launch_bounds__(kTThreads, 4) post_v_kernel(const PostParams p
 #pragma unroll
     for (int j = 0; j < kAhead; ++j) {
         const float4* at = hdr + (size_t)(ys + j) * W + x;
-        us[j] = ys + j < H ? __ldg(at) : zero;
-        vs[j] = ys + j < H && second ? __ldg(at + 1) : zero;
+        us[j] = ys + j < H ? load_behind_wait(at) : zero;
+        vs[j] = ys + j < H && second ? load_behind_wait(at + 1) : zero;
     }
 #pragma unroll
     for (int j = 0; j < kBJ; ++j) {
@@ -981,8 +990,8 @@ __global__ void __launch_bounds__(kTThreads, 4) post_v_kernel(const PostParams p
         const float4 u = us[j % kAhead], v = vs[j % kAhead];
         if (j + kAhead < kBJ) {
             const float4* at = hdr + (size_t)(y + kAhead) * W + x;
-            us[j % kAhead] = y + kAhead < H ? __ldg(at) : zero;
-            vs[j % kAhead] = y + kAhead < H && second ? __ldg(at + 1) : zero;
+            us[j % kAhead] = y + kAhead < H ? load_behind_wait(at) : zero;
+            vs[j % kAhead] = y + kAhead < H && second ? load_behind_wait(at + 1) : zero;
         }
         image[idx] = tone_pack(u.x + lo2(acc[j][0]) * pp.intensity, u.y + lo2(acc[j][1]) * pp.intensity,
                                u.z + lo2(acc[j][2]) * pp.intensity);
@@ -1091,8 +1100,7 @@ static cudaError_t launch_h(const PostParams& pp, const float4* hdr, float4* blo
     const cudaError_t e = set_smem((const void*)bloom_h_kernel<PAIRED>, sm);
     if (e != cudaSuccess) return e;
     const dim3 grid((pp.width + kTPos - 1) / kTPos, (pp.height + 2 * kTPairs - 1) / (2 * kTPairs));
-    bloom_h_kernel<PAIRED><<<grid, kTThreads, sm, st>>>(pp, hdr, bloom);
-    return cudaGetLastError();
+    return launch_early(bloom_h_kernel<PAIRED>, grid, kTThreads, sm, st, pp, hdr, bloom);
 }
 template <bool PAIRED>
 static cudaError_t launch_v(const PostParams& pp, const float4* hdr, const float4* bloom, uint32_t* image,
@@ -1101,8 +1109,7 @@ static cudaError_t launch_v(const PostParams& pp, const float4* hdr, const float
     const cudaError_t e = set_smem((const void*)post_v_kernel<PAIRED>, sm);
     if (e != cudaSuccess) return e;
     const dim3 grid((pp.width + 2 * kTPairs - 1) / (2 * kTPairs), (pp.height + kTPos - 1) / kTPos);
-    post_v_kernel<PAIRED><<<grid, kTThreads, sm, st>>>(pp, hdr, bloom, image);
-    return cudaGetLastError();
+    return launch_early(post_v_kernel<PAIRED>, grid, kTThreads, sm, st, pp, hdr, bloom, image);
 }
 
 cudaError_t launch_bloom_horizontal(const PostParams& pp, const float4* hdr, float4* bloom, cudaStream_t st) {

@@ -184,3 +184,50 @@ def test_post_tiles_against_oracle(cuda, orc, size, radius):
                       np.stack([(exp >> s) & 255 for s in (16, 8, 0)]).astype(int)), axis=0)
     assert d.max() <= 1, np.bincount(d)
     ctx.close()
+
+
+@pytest.mark.parametrize("size,radius", [((33, 17), 2.0), ((333, 217), 24.0), ((960, 540), 24.0)])
+@pytest.mark.parametrize("graph", [False, True])
+def test_overlapped_launches_keep_stream_order(cuda, size, radius, graph):
+    """Post passes issued one behind the other on two streams, each behind a kernel or a copy that
+    rewrites its input (directly and as one captured graph), equal the passes run one at a time."""
+    cfg, _ = workloads.scene("t1")
+    cfg = workloads.scaled(cfg, *size)
+    cfg.bloom_radius = radius
+    n = size[0] * size[1]
+    inputs = [_hdr_input(cuda, cfg, 11 + i) for i in range(3)]
+    ctx = [kt.Context(cfg) for _ in range(2)]
+    hdr = [cuda.zeros((n, 4), device="cuda") for _ in ctx]
+    img = [cuda.zeros(n, dtype=cuda.int32, device="cuda") for _ in ctx]
+    want = []
+    for x in inputs:
+        ctx[0].post_fused(x.data_ptr(), img[0].data_ptr())
+        cuda.cuda.synchronize()
+        want.append(img[0].clone())
+    got = [[cuda.zeros_like(i) for _ in range(12)] for i in img]
+
+    def issue(q, stream):
+        for it in range(12):
+            x = inputs[(it + q) % 3]
+            (cuda.mul(x, 1.0, out=hdr[q]) if it % 2 else hdr[q].copy_(x))
+            ctx[q].post_fused(hdr[q].data_ptr(), img[q].data_ptr(), stream.cuda_stream)
+            got[q][it].copy_(img[q])
+
+    streams = [cuda.cuda.Stream() for _ in ctx]
+    graphs = []
+    cuda.cuda.synchronize()
+    for q, st in enumerate(streams):
+        if graph:
+            g = cuda.cuda.CUDAGraph()
+            with cuda.cuda.graph(g, stream=st):
+                issue(q, st)
+            graphs.append(g)
+        else:
+            with cuda.cuda.stream(st):
+                issue(q, st)
+    for g in graphs:
+        g.replay()
+    cuda.cuda.synchronize()
+    for q in range(2):
+        for it in range(12):
+            assert cuda.equal(got[q][it], want[(it + q) % 3]), (q, it)
