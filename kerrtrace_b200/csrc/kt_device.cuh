@@ -125,6 +125,52 @@ template <class R> struct DP {
     static constexpr R d7 = R(69997945.0) / R(29380423.0);
 };
 
+// ---- pairs of floats ------------------------------------------------------------------------
+__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
+    return (uint64_t)__float_as_uint(lo) | (uint64_t)__float_as_uint(hi) << 32;
+}
+__device__ __forceinline__ float lo2(uint64_t v) { return __uint_as_float((unsigned)v); }
+__device__ __forceinline__ float hi2(uint64_t v) { return __uint_as_float((unsigned)(v >> 32)); }
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t r;
+    asm("fma.rn.ftz.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("mul.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+// Stage sums of the mixed tracer on pairs of components: out = w[0] k[0] + w[1] k[1] + ..., with the
+// second product rounded and the others added by multiply-adds, first, third, fourth: the bits of
+// the scalar sum as the compiler contracts it.
+//
+// Why: the mixed kernel issued on 83% of cycles with its FP32 pipe 68% busy, and these sums are a
+// fifth of its multiply-adds.  A packed one holds the pipe as long as two plain ones but takes
+// one issue slot: 1024^2 at 1 sample 1147 -> 1087 us (persistent), 1117 -> 1098 (tuned plain).  The
+// FP32 tracers keep the scalar sums: their pipe is full at 77%, so packing takes 9% off their
+// instructions and nothing off their time (1920x1080 2.21 -> 2.19 ms persistent, 2.19 -> 2.23 plain).
+template <int N>
+__device__ __forceinline__ void weigh(float (&out)[6], const float (&w)[N], const float* const (&k)[N]) {
+#pragma unroll
+    for (int c = 0; c < 6; c += 2) {
+        uint64_t acc = mul2(pack2(w[1], w[1]), pack2(k[1][c], k[1][c + 1]));
+#pragma unroll
+        for (int i = 0; i < N; ++i)
+            if (i != 1) acc = fma2(pack2(w[i], w[i]), pack2(k[i][c], k[i][c + 1]), acc);
+        out[c] = lo2(acc);
+        out[c + 1] = hi2(acc);
+    }
+}
+__device__ __forceinline__ void step_to(float (&y)[6], const float* s, float h, const float* d) {
+#pragma unroll
+    for (int c = 0; c < 6; c += 2) {
+        const uint64_t v = fma2(pack2(h, h), pack2(d[c], d[c + 1]), pack2(s[c], s[c + 1]));
+        y[c] = lo2(v);
+        y[c + 1] = hi2(v);
+    }
+}
+
 // ---- PCG hash (cuda/kerr_math.cuh:26-36) ------------------------------------------------
 __device__ __forceinline__ uint32_t pcg_hash(uint64_t state) {
     const uint64_t x = state * 6364136223846793005ULL + 1442695040888963407ULL;

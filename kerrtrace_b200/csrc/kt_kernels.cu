@@ -658,18 +658,10 @@ __device__ __forceinline__ PairTile pair_tile(void* smem, int R) {
     return t;
 }
 
-__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
-    return (uint64_t)__float_as_uint(lo) | (uint64_t)__float_as_uint(hi) << 32;
-}
-__device__ __forceinline__ float lo2(uint64_t v) { return __uint_as_float((unsigned)v); }
-__device__ __forceinline__ float hi2(uint64_t v) { return __uint_as_float((unsigned)(v >> 32)); }
-__device__ __forceinline__ void fma2(uint64_t& acc, uint64_t v, uint64_t w) {
-    asm("fma.rn.ftz.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(v), "l"(w));
-}
 __device__ __forceinline__ void tap2(uint64_t (&acc)[3], const ulonglong2& rg, uint64_t b, uint64_t w) {
-    fma2(acc[0], rg.x, w);
-    fma2(acc[1], rg.y, w);
-    fma2(acc[2], b, w);
+    acc[0] = fma2(rg.x, w, acc[0]);
+    acc[1] = fma2(rg.y, w, acc[1]);
+    acc[2] = fma2(b, w, acc[2]);
 }
 
 // kBJ outputs of one pair; rg, b: the thread's first source.
@@ -758,15 +750,6 @@ __device__ __forceinline__ void load_row_pair(const float4* row, int W, float4 (
             v[q] = load_behind_wait(row + W + 32 * q);
         }
     }
-}
-
-// A pair of blurred values over the sum of their in-image weights (cuda/kernel.cu:167-171, 210-214), whose
-// reciprocal the tables hold: the fast division is that product (and no division where the sum
-// is 0: the tables hold 1).
-__device__ __forceinline__ uint64_t scale2(uint64_t v, uint64_t s) {
-    uint64_t r;
-    asm("mul.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r) : "l"(v), "l"(s));
-    return r;
 }
 
 // Asynchronous copies global -> shared (cp.async); the bytes past src_bytes are zero-filled and
@@ -860,11 +843,13 @@ __global__ void __launch_bounds__(kTThreads, 5) bloom_h_kernel(const PostParams 
     uint64_t acc[kBJ][3];
     blur_pair(t.rg + p * stride + cb, t.b + p * stride + cb, t.w, R, acc);
     const int xs = x0 + cb, y = y0 + 2 * p;
+    // over the sum of the in-image weights (cuda/kernel.cu:167-171, 210-214), whose reciprocal the
+    // tables hold: the fast division is that product (no division where the sum is 0: they hold 1)
 #pragma unroll
     for (int j = 0; j < kBJ; ++j) {
         const float s = t.inv[cb + j];
 #pragma unroll
-        for (int c = 0; c < 3; ++c) acc[j][c] = scale2(acc[j][c], pack2(s, s));
+        for (int c = 0; c < 3; ++c) acc[j][c] = mul2(acc[j][c], pack2(s, s));
     }
     if (PAIRED) {
         float4* rg = bloom;
@@ -986,7 +971,7 @@ __global__ void __launch_bounds__(kTThreads, 4) post_v_kernel(const PostParams p
         const size_t idx = (size_t)y * W + x;
         const float s = t.inv[cb + j];
 #pragma unroll
-        for (int c = 0; c < 3; ++c) acc[j][c] = scale2(acc[j][c], pack2(s, s));
+        for (int c = 0; c < 3; ++c) acc[j][c] = mul2(acc[j][c], pack2(s, s));
         const float4 u = us[j % kAhead], v = vs[j % kAhead];
         if (j + kAhead < kBJ) {
             const float4* at = hdr + (size_t)(y + kAhead) * W + x;

@@ -673,28 +673,22 @@ __device__ __forceinline__ int ray_advance_mixed(RayRun<Mixed>& ry, const Scene&
     const float* s = ry.s;
     const float* k1 = ry.k1;
     float y[6], k2[6], k3[6], k4[6], k5[6], k6[6], k7[6], nx[6], inc[6];
-#pragma unroll
-    for (int c = 0; c < 6; ++c) y[c] = s[c] + h * C::a21 * k1[c];
+    step_to(y, s, h * C::a21, k1);
     hamilton_rhs<float, EXACT>(y, pt, a, aa, M, k2);
-#pragma unroll
-    for (int c = 0; c < 6; ++c) y[c] = s[c] + h * (C::a31 * k1[c] + C::a32 * k2[c]);
+    weigh<2>(inc, {C::a31, C::a32}, {k1, k2});
+    step_to(y, s, h, inc);
     hamilton_rhs<float, EXACT>(y, pt, a, aa, M, k3);
-#pragma unroll
-    for (int c = 0; c < 6; ++c) y[c] = s[c] + h * (C::a41 * k1[c] + C::a42 * k2[c] + C::a43 * k3[c]);
+    weigh<3>(inc, {C::a41, C::a42, C::a43}, {k1, k2, k3});
+    step_to(y, s, h, inc);
     hamilton_rhs<float, EXACT>(y, pt, a, aa, M, k4);
-#pragma unroll
-    for (int c = 0; c < 6; ++c)
-        y[c] = s[c] + h * (C::a51 * k1[c] + C::a52 * k2[c] + C::a53 * k3[c] + C::a54 * k4[c]);
+    weigh<4>(inc, {C::a51, C::a52, C::a53, C::a54}, {k1, k2, k3, k4});
+    step_to(y, s, h, inc);
     hamilton_rhs<float, EXACT>(y, pt, a, aa, M, k5);
-#pragma unroll
-    for (int c = 0; c < 6; ++c)
-        y[c] = s[c] + h * (C::a61 * k1[c] + C::a62 * k2[c] + C::a63 * k3[c] + C::a64 * k4[c] + C::a65 * k5[c]);
+    weigh<5>(inc, {C::a61, C::a62, C::a63, C::a64, C::a65}, {k1, k2, k3, k4, k5});
+    step_to(y, s, h, inc);
     hamilton_rhs<float, EXACT>(y, pt, a, aa, M, k6);
-#pragma unroll
-    for (int c = 0; c < 6; ++c) {
-        inc[c] = C::b1 * k1[c] + C::b3 * k3[c] + C::b4 * k4[c] + C::b5 * k5[c] + C::b6 * k6[c];
-        nx[c] = s[c] + h * inc[c];
-    }
+    weigh<5>(inc, {C::b1, C::b3, C::b4, C::b5, C::b6}, {k1, k3, k4, k5, k6});
+    step_to(nx, s, h, inc);
     hamilton_rhs<float, EXACT>(nx, pt, a, aa, M, k7);
     float errv;
     const bool going = !TOGETHER || state == kRayGoing;
@@ -717,11 +711,11 @@ __device__ __forceinline__ int ray_advance_mixed(RayRun<Mixed>& ry, const Scene&
         errv = any ? (float)em : __int_as_float(0x7fffffff);
     } else {
         float e[6];
+        weigh<6>(e, {C::e1, C::e3, C::e4, C::e5, C::e6, C::e7}, {k1, k3, k4, k5, k6, k7});
 #pragma unroll
         for (int c = 0; c < 6; ++c) {
             const float scale = ry.tol * O::maxr(O::absr(s[c]), 1.0f);
-            e[c] = O::absr(h * (C::e1 * k1[c] + C::e3 * k3[c] + C::e4 * k4[c] + C::e5 * k5[c] + C::e6 * k6[c] +
-                                C::e7 * k7[c])) / scale;
+            e[c] = O::absr(h * e[c]) / scale;
         }
         errv = O::maxr(O::maxr(O::maxr(e[0], e[1]), O::maxr(e[2], e[3])), O::maxr(e[4], e[5]));
     }
