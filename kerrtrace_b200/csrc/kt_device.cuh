@@ -141,15 +141,19 @@ __device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
     asm("mul.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
     return r;
 }
-// Stage sums of the mixed tracer on pairs of components: out = w[0] k[0] + w[1] k[1] + ..., with the
-// second product rounded and the others added by multiply-adds, first, third, fourth: the bits of
-// the scalar sum as the compiler contracts it.
+// Stage sums on pairs of components: out = w[0] k[0] + w[1] k[1] + ..., with the second product
+// rounded and the others added by multiply-adds, first, third, fourth: the bits of the scalar sum as
+// the compiler contracts it.
 //
-// Why: the mixed kernel issued on 83% of cycles with its FP32 pipe 68% busy, and these sums are a
-// fifth of its multiply-adds.  A packed one holds the pipe as long as two plain ones but takes
-// one issue slot: 1024^2 at 1 sample 1147 -> 1087 us (persistent), 1117 -> 1098 (tuned plain).  The
-// FP32 tracers keep the scalar sums: their pipe is full at 77%, so packing takes 9% off their
-// instructions and nothing off their time (1920x1080 2.21 -> 2.19 ms persistent, 2.19 -> 2.23 plain).
+// Why: a packed multiply-add holds the FP32 pipe as long as two plain ones but takes one issue slot,
+// and these sums are a fifth of an attempt's multiply-adds.  Kernels that run out of slots first
+// gain: mixed (issuing on 83% of cycles, pipe 68% busy) 1024^2 1147 -> 1087 us persistent, 1117 -> 1098
+// tuned plain; stated physics 1920x1080 2.36 -> 2.24 ms persistent, 2.167 -> 2.159 plain, its recording
+// forward at 512^2 392 -> 374 us; eight 480x270 views without textures 1247 -> 1217.  The FP32
+// reference tracer keeps the scalar sums: its pipe is full at 77%, so packing takes 9% off its
+// instructions and nothing off its time (1920x1080 2.21 -> 2.19 ms persistent, 2.19 -> 2.23 plain).
+// So do the FP32 launches of one unit per warp, which wait for latencies and not for slots (a
+// 48x27 view 107.5 us, packed 109.6).
 template <int N>
 __device__ __forceinline__ void weigh(float (&out)[6], const float (&w)[N], const float* const (&k)[N]) {
 #pragma unroll

@@ -391,6 +391,32 @@ __device__ __forceinline__ void ray_sky(RayRun<R>& ry, const Scene& sc, Tally& t
     ry.col[2] += sky;
 }
 
+// The stages of an attempt from s and k1 on pairs of components; inc is the weighted sum of the step.
+template <bool EXACT>
+__device__ __forceinline__ void stages_packed(const float* s, const float* k1, float h, float pt, float a, float aa,
+                                              float M, float (&k2)[6], float (&k3)[6], float (&k4)[6], float (&k5)[6],
+                                              float (&k6)[6], float (&k7)[6], float (&nx)[6], float (&inc)[6]) {
+    using C = DP<float>;
+    float y[6];
+    step_to(y, s, h * C::a21, k1);
+    hamilton_rhs<float, EXACT>(y, pt, a, aa, M, k2);
+    weigh<2>(inc, {C::a31, C::a32}, {k1, k2});
+    step_to(y, s, h, inc);
+    hamilton_rhs<float, EXACT>(y, pt, a, aa, M, k3);
+    weigh<3>(inc, {C::a41, C::a42, C::a43}, {k1, k2, k3});
+    step_to(y, s, h, inc);
+    hamilton_rhs<float, EXACT>(y, pt, a, aa, M, k4);
+    weigh<4>(inc, {C::a51, C::a52, C::a53, C::a54}, {k1, k2, k3, k4});
+    step_to(y, s, h, inc);
+    hamilton_rhs<float, EXACT>(y, pt, a, aa, M, k5);
+    weigh<5>(inc, {C::a61, C::a62, C::a63, C::a64, C::a65}, {k1, k2, k3, k4, k5});
+    step_to(y, s, h, inc);
+    hamilton_rhs<float, EXACT>(y, pt, a, aa, M, k6);
+    weigh<5>(inc, {C::b1, C::b3, C::b4, C::b5, C::b6}, {k1, k3, k4, k5, k6});
+    step_to(nx, s, h, inc);
+    hamilton_rhs<float, EXACT>(nx, pt, a, aa, M, k7);
+}
+
 // One DP5(4) attempt; on the last attempt of a step, the commit and the per-step tests.
 // TOGETHER (run_rays): the ray may already have ended (its attempt is computed and dropped), and
 // the sky of an escaped ray is left to the caller.
@@ -398,44 +424,55 @@ template <class R, int MODE, bool COUNT, bool TOGETHER>
 __device__ __forceinline__ int ray_advance(RayRun<R>& ry, const Scene& sc, uint32_t* err,
                                            Tally& tl, int state) {
     constexpr bool EXACT = MODE == 1;
+    constexpr bool PACKED = std::is_same<R, float>::value && MODE != 0 && !TOGETHER;
     using O = Ops<R>;
     using C = DP<R>;
     const R a = sc_a<R>(sc), aa = sc_aa<R>(sc), M = sc_M<R>(sc);
     const R h = ry.h;
     const R* s = ry.s;
     const R* k1 = ry.k1;
-    R y[6], k2[6], k3[6], k4[6], k5[6], k6[6], k7[6], nx[6];
+    R k2[6], k3[6], k4[6], k5[6], k6[6], k7[6], nx[6];
+    if constexpr (PACKED) {
+        R inc[6];
+        stages_packed<EXACT>(s, k1, h, ry.pt, a, aa, M, k2, k3, k4, k5, k6, k7, nx, inc);
+    } else {
+        R y[6];
 #pragma unroll
-    for (int c = 0; c < 6; ++c) y[c] = s[c] + h * C::a21 * k1[c];
-    hamilton_rhs<R, EXACT>(y, ry.pt, a, aa, M, k2);
+        for (int c = 0; c < 6; ++c) y[c] = s[c] + h * C::a21 * k1[c];
+        hamilton_rhs<R, EXACT>(y, ry.pt, a, aa, M, k2);
 #pragma unroll
-    for (int c = 0; c < 6; ++c) y[c] = s[c] + h * (C::a31 * k1[c] + C::a32 * k2[c]);
-    hamilton_rhs<R, EXACT>(y, ry.pt, a, aa, M, k3);
+        for (int c = 0; c < 6; ++c) y[c] = s[c] + h * (C::a31 * k1[c] + C::a32 * k2[c]);
+        hamilton_rhs<R, EXACT>(y, ry.pt, a, aa, M, k3);
 #pragma unroll
-    for (int c = 0; c < 6; ++c) y[c] = s[c] + h * (C::a41 * k1[c] + C::a42 * k2[c] + C::a43 * k3[c]);
-    hamilton_rhs<R, EXACT>(y, ry.pt, a, aa, M, k4);
+        for (int c = 0; c < 6; ++c) y[c] = s[c] + h * (C::a41 * k1[c] + C::a42 * k2[c] + C::a43 * k3[c]);
+        hamilton_rhs<R, EXACT>(y, ry.pt, a, aa, M, k4);
 #pragma unroll
-    for (int c = 0; c < 6; ++c)
-        y[c] = s[c] + h * (C::a51 * k1[c] + C::a52 * k2[c] + C::a53 * k3[c] + C::a54 * k4[c]);
-    hamilton_rhs<R, EXACT>(y, ry.pt, a, aa, M, k5);
+        for (int c = 0; c < 6; ++c)
+            y[c] = s[c] + h * (C::a51 * k1[c] + C::a52 * k2[c] + C::a53 * k3[c] + C::a54 * k4[c]);
+        hamilton_rhs<R, EXACT>(y, ry.pt, a, aa, M, k5);
 #pragma unroll
-    for (int c = 0; c < 6; ++c)
-        y[c] = s[c] + h * (C::a61 * k1[c] + C::a62 * k2[c] + C::a63 * k3[c] + C::a64 * k4[c] +
-                           C::a65 * k5[c]);
-    hamilton_rhs<R, EXACT>(y, ry.pt, a, aa, M, k6);
-    // 5th-order solution; its stage-7 input is the same expression (a7j = b_j), so k7 is FSAL
+        for (int c = 0; c < 6; ++c)
+            y[c] = s[c] + h * (C::a61 * k1[c] + C::a62 * k2[c] + C::a63 * k3[c] + C::a64 * k4[c] +
+                               C::a65 * k5[c]);
+        hamilton_rhs<R, EXACT>(y, ry.pt, a, aa, M, k6);
+        // 5th-order solution; its stage-7 input is the same expression (a7j = b_j), so k7 is FSAL
 #pragma unroll
-    for (int c = 0; c < 6; ++c)
-        nx[c] = s[c] + h * (C::b1 * k1[c] + C::b3 * k3[c] + C::b4 * k4[c] + C::b5 * k5[c] +
-                            C::b6 * k6[c]);
-    hamilton_rhs<R, EXACT>(nx, ry.pt, a, aa, M, k7);
+        for (int c = 0; c < 6; ++c)
+            nx[c] = s[c] + h * (C::b1 * k1[c] + C::b3 * k3[c] + C::b4 * k4[c] + C::b5 * k5[c] +
+                                C::b6 * k6[c]);
+        hamilton_rhs<R, EXACT>(nx, ry.pt, a, aa, M, k7);
+    }
     // max-norm of the embedded error, per-component scale tol * max(|y_i|, 1)
     R e[6];
+    if constexpr (PACKED) weigh<6>(e, {C::e1, C::e3, C::e4, C::e5, C::e6, C::e7}, {k1, k3, k4, k5, k6, k7});
 #pragma unroll
     for (int c = 0; c < 6; ++c) {
         const R scale = ry.tol * O::maxr(O::absr(s[c]), R(1));
-        e[c] = O::ratio(O::absr(h * (C::e1 * k1[c] + C::e3 * k3[c] + C::e4 * k4[c] + C::e5 * k5[c] +
-                                     C::e6 * k6[c] + C::e7 * k7[c])), scale);
+        if constexpr (PACKED)
+            e[c] = O::ratio(O::absr(h * e[c]), scale);
+        else
+            e[c] = O::ratio(O::absr(h * (C::e1 * k1[c] + C::e3 * k3[c] + C::e4 * k4[c] + C::e5 * k5[c] +
+                                         C::e6 * k6[c] + C::e7 * k7[c])), scale);
     }
     R errv = O::maxr(O::maxr(O::maxr(e[0], e[1]), O::maxr(e[2], e[3])), O::maxr(e[4], e[5]));
     if constexpr (std::is_same<R, double>::value) {
@@ -672,24 +709,8 @@ __device__ __forceinline__ int ray_advance_mixed(RayRun<Mixed>& ry, const Scene&
     const float h = ry.h;
     const float* s = ry.s;
     const float* k1 = ry.k1;
-    float y[6], k2[6], k3[6], k4[6], k5[6], k6[6], k7[6], nx[6], inc[6];
-    step_to(y, s, h * C::a21, k1);
-    hamilton_rhs<float, EXACT>(y, pt, a, aa, M, k2);
-    weigh<2>(inc, {C::a31, C::a32}, {k1, k2});
-    step_to(y, s, h, inc);
-    hamilton_rhs<float, EXACT>(y, pt, a, aa, M, k3);
-    weigh<3>(inc, {C::a41, C::a42, C::a43}, {k1, k2, k3});
-    step_to(y, s, h, inc);
-    hamilton_rhs<float, EXACT>(y, pt, a, aa, M, k4);
-    weigh<4>(inc, {C::a51, C::a52, C::a53, C::a54}, {k1, k2, k3, k4});
-    step_to(y, s, h, inc);
-    hamilton_rhs<float, EXACT>(y, pt, a, aa, M, k5);
-    weigh<5>(inc, {C::a61, C::a62, C::a63, C::a64, C::a65}, {k1, k2, k3, k4, k5});
-    step_to(y, s, h, inc);
-    hamilton_rhs<float, EXACT>(y, pt, a, aa, M, k6);
-    weigh<5>(inc, {C::b1, C::b3, C::b4, C::b5, C::b6}, {k1, k3, k4, k5, k6});
-    step_to(nx, s, h, inc);
-    hamilton_rhs<float, EXACT>(nx, pt, a, aa, M, k7);
+    float k2[6], k3[6], k4[6], k5[6], k6[6], k7[6], nx[6], inc[6];
+    stages_packed<EXACT>(s, k1, h, pt, a, aa, M, k2, k3, k4, k5, k6, k7, nx, inc);
     float errv;
     const bool going = !TOGETHER || state == kRayGoing;
     if (COUNT && ry.zone && going) tl.fp64++;
