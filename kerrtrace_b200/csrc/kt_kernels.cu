@@ -363,7 +363,15 @@ static cudaError_t launch_wave_minb(const Scene& sc, const Camera& cam, float4* 
     const int S = samples_in_parallel(sc.spp);
     const unsigned units = unit_count(sc.width, sc.height, S, order != nullptr);
     const unsigned blocks = (units + kWarps - 1) / kWarps, resident = (unsigned)(sms * MINB);
-    const unsigned grid = blocks < resident ? blocks : resident;
+    // Stated physics in FP32 and FP64: a block per four units, not only the resident ones.  The
+    // hardware's block scheduler then hands out the units and the warps of a block start
+    // together, at the same place of a loop body (30 KB in FP64) that outgrows the nearer instruction
+    // caches; persistent warps drift apart and the FP64 kernel waited for instructions 0.7
+    // cycles per issue.  960x540 FP64 3.24 -> 2.99 ms, 1920x1080 6.58 -> 5.75, 400x300 x 3 samples 2.89 ->
+    // 2.66; 1920x1080 FP32 2.16-2.36 -> 2.08.  The mixed and the reference trace gain nothing (1.088 ->
+    // 1.097, 2.217 -> 2.227) and stay persistent.
+    constexpr bool kAllBlocks = MODE == 1 && !std::is_same<R, Mixed>::value;
+    const unsigned grid = kAllBlocks || blocks < resident ? blocks : resident;
     if (units > grid * kWarps) {
         e = cudaMemsetAsync(queue, 0, sizeof(unsigned), st);
         if (e != cudaSuccess) return e;

@@ -44,7 +44,7 @@ constexpr int kNoallocBlock = 128;
 // Persistent trace over several views of one scene, in the units of trace_wavefront_kernel: 32 / S
 // pixels with S samples of each side by side, view after view.  A warp's first unit is its own index
 // in the grid, the others come from one counter over all views.  (Refilling single lanes, as an
-// earlier form did, ran the ray set-up for one lane of 32: 8 views of 480x270 1.78 ms, now 1.26; at
+// earlier form did, ran the ray set-up for one lane of 32: 8 views of 480x270 1.78 ms, now 1.22; at
 // 4 samples 8.55, now 4.59; 12 views of 64x36 at 2 samples 418 us, now 162.)
 template <bool TOGETHER>
 __global__ void __launch_bounds__(kNoallocBlock, 4)
