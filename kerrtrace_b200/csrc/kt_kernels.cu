@@ -491,7 +491,8 @@ cudaError_t launch_batch(const BatchTable& bt, int bx, int by, cudaStream_t st) 
 // patch holds rays more alike than one of 16x2: 64 renders of 128x128 to 960x540 15.75 -> 15.45
 // ms, 64 up to 400x225 3.01 -> 2.95.  A batch of one unit per warp at most lasts as long as its
 // longest ray, and takes the loop that keeps a warp's lanes in step (TOGETHER): two renders of
-// 100 columns 130 -> 104 us, five of up to 160 181 -> 130.
+// 100 columns 130 -> 104 us, five of up to 160 181 -> 130.  In FP64 every unit gets its warp at the launch
+// (64 renders of 64x64 to 480x270: 12.16 -> 11.24 ms; stated FP32 3.27 -> 3.37, so it does not).
 template <class R, int MODE, int MINB, bool TOGETHER>
 __global__ void __launch_bounds__(kWavefrontBlock, MINB)
     trace_batch_persistent_kernel(const __grid_constant__ BatchTable bt, unsigned* __restrict__ counter) {
@@ -537,6 +538,11 @@ static cudaError_t launch_batch_persistent_minb(const BatchTable& bt, unsigned* 
     if (bt.total_units <= warps) {
         const unsigned blocks = (bt.total_units + kWavefrontBlock / 32 - 1) / (kWavefrontBlock / 32);
         trace_batch_persistent_kernel<R, MODE, MINB, true><<<blocks, kWavefrontBlock, 0, st>>>(bt, counter);
+        return cudaGetLastError();
+    }
+    if (std::is_same<R, double>::value) {  // a block per four units, as the single frame (launch_wave_minb)
+        const unsigned blocks = (bt.total_units + kWavefrontBlock / 32 - 1) / (kWavefrontBlock / 32);
+        trace_batch_persistent_kernel<R, MODE, MINB, false><<<blocks, kWavefrontBlock, 0, st>>>(bt, counter);
         return cudaGetLastError();
     }
     if ((e = cudaMemsetAsync(counter, 0, sizeof(unsigned), st)) != cudaSuccess) return e;
