@@ -57,10 +57,14 @@ typedef enum kt_mode { KT_MODE_REF = 0, KT_MODE_SPEC = 1 } kt_mode;
  * solve.  FP64 runs the whole integration in double. */
 typedef enum kt_precision { KT_PREC_FP32 = 0, KT_PREC_MIXED = 1, KT_PREC_FP64 = 2 } kt_precision;
 
-/* Scheduling of the trace kernel.  All schedules produce the same image bits. */
+/* Scheduling of the trace kernel.  All schedules produce the same image bits at one sample per pixel.
+ * With more, the reference-semantics wavefront kernel rounds one product of a later sample's ray
+ * start the other way round, so a few rays of some cameras differ from the plain schedule by an ulp
+ * there. */
 typedef enum kt_schedule {
     KT_SCHED_PLAIN = 0,     /* one thread per pixel on a 2D grid of block_dim tiles (kernel.cu:88) */
-    KT_SCHED_WAVEFRONT = 1, /* persistent kernel, warps take units of 32 rays from a work counter */
+    KT_SCHED_WAVEFRONT = 1, /* warps take units of 32 rays: a persistent kernel whose warps draw further units
+                               from a work counter, or (stated physics, FP32 and FP64) a warp per unit */
     KT_SCHED_AUTO = 2       /* whichever the context's kt_tuning selects (the autotuner's choice) */
 } kt_schedule;
 
@@ -344,8 +348,8 @@ uint64_t kt_batch_rays(const kt_batch* b);
 void kt_batch_destroy(kt_batch* b);
 
 /* ---- trace without any device allocation --------------------------------------------------- */
-/* Largest n_views of one kt_trace_noalloc call: its scratch is one 32-bit work counter per view,
- * held in a 256-byte array inside the library's device image. */
+/* Largest n_views of one kt_trace_noalloc call.  Its scratch is a 32-bit work counter over all views, in a
+ * 256-byte array inside the library's device image. */
 #define KT_NOALLOC_MAX_VIEWS 64
 /*
  * No counterpart in the reference.  For callers that cannot allocate device memory where they

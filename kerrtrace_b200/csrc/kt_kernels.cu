@@ -7,8 +7,9 @@
 // Trace kernels (replace trace_kernel, cuda/kernel.cu:88-142):
 //   trace_plain_kernel      one thread per pixel on a 2D grid of block_dim tiles; each thread
 //                           runs its spp rays to completion through the attempt state machine.
-//   trace_wavefront_kernel  persistent: one block per resident slot, each warp takes units of 32
-//                           rays (pixels x samples) from a device work counter.
+//   trace_wavefront_kernel  warps take units of 32 rays (pixels x samples): persistent warps, the first
+//                           unit by index and the others from a device work counter, or a warp
+//                           per unit.
 // Post kernels (replace bloom_horizontal / post_process, cuda/kernel.cu:144-251):
 //   bloom_h_kernel          horizontal normalised Gaussian over tiles staged in pairs of rows
 //   post_v_kernel           vertical Gaussian over tiles staged in pairs of columns + composite,
@@ -250,7 +251,7 @@ __global__ void __launch_bounds__(MAXT, MINB)
 // post, default tuning): 1920x1080 reference 3.58 -> 2.30 ms (trace), 960x540 FP64 6.69 -> 4.39,
 // 1024^2 mixed 2.62 -> 1.70, two frames of 2100x900 at 4 samples 15.9 -> 7.39; 96x64 at 2 samples
 // 0.272 -> 0.098, where a pixel's samples used to run one after the other on one lane; with
-// frozen rays kept to the end 183 -> 173.
+// frozen rays kept to the end (a switch for timing) 183 -> 187.
 template <class R, int MODE, bool COUNT, int MINB, bool TOGETHER>
 __global__ void __launch_bounds__(kWavefrontBlock, MINB)
     trace_wavefront_kernel(const __grid_constant__ Scene sc, const Camera cam, float4* __restrict__ hdr,
