@@ -248,9 +248,9 @@ __global__ void __launch_bounds__(MAXT, MINB)
 // of their own unit finish.  An earlier form refilled single lanes from the counter as their
 // rays ended: each refill ran the start-up code (ray set-up, first tolerance, first right-hand
 // side) for one lane of 32, which cost more than the idle lanes it filled.  Against it (trace and
-// post, default tuning): 1920x1080 reference 3.58 -> 2.30 ms (trace), 960x540 FP64 6.69 -> 4.39,
-// 1024^2 mixed 2.62 -> 1.70, two frames of 2100x900 at 4 samples 15.9 -> 7.39; 96x64 at 2 samples
-// 0.272 -> 0.098, where a pixel's samples used to run one after the other on one lane; with
+// post, default tuning; with the later steps in it): 1920x1080 reference 3.58 -> 2.21 ms (trace),
+// 960x540 FP64 5.67 -> 2.42, 1024^2 mixed 2.64 -> 1.09, two frames of 2100x900 at 4 samples 16.0 -> 7.16;
+// 96x64 at 2 samples 0.277 -> 0.080, where a pixel's samples used to run one after the other on one lane; with
 // frozen rays kept to the end (a switch for timing) 183 -> 187.
 template <class R, int MODE, bool COUNT, int MINB, bool TOGETHER>
 __global__ void __launch_bounds__(kWavefrontBlock, MINB)
