@@ -113,7 +113,7 @@ struct BatchTable {
 };
 cudaError_t launch_batch(const BatchTable& bt, int bx, int by, cudaStream_t stream);
 // Persistent batched trace: warps take 32-pixel units, each inside one job, from the device
-// counter `counter` (one word, reset here on `stream`); blocks of 128 threads, blocks_per_sm
+// counter `counter` (one word, reset here on `stream` when it is used); blocks of 128 threads, blocks_per_sm
 // resident per SM (the FP32 reference-semantics kernel has 4, 5 and 6; the others their default).
 cudaError_t launch_batch_persistent(const BatchTable& bt, int blocks_per_sm, unsigned* counter, cudaStream_t stream);
 // Number of 16-byte words that differ between a and b (n16 words each) into *out (device).
