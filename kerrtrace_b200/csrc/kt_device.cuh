@@ -44,22 +44,36 @@ template <> struct Ops<float> {
     static __device__ __forceinline__ bool isnanr(float a) { return isnan(a); }
     static __device__ __forceinline__ bool isfiniter(float a) { return isfinite(a); }
 };
-// Double division and square root round correctly like the operators, but without their branches: an
-// attempt holds 22 divisions, and each branch to a slow path ends the block that the compiler can
-// overlap, so a warp waited out one division after the other.  1/b is Markstein's: rcp.approx (about
-// 20 bits), one third-order step (e + e^2 with e = 1 - b y), and a last Newton step on an estimate
-// within an ulp, which rounds correctly; a/b adds his remainder step.  The square root takes the same
-// last step (s + y/2 (x - s^2)).  They hold for operands and results in the normal range; zero,
-// infinite and NaN divisors give NaN.  No result of 268 million random operands (e^-30 .. e^30)
-// differed from the operators'; c2 view in FP64, tuned plain shape: 960x540 3.43 -> 2.63 ms,
-// 1920x1080 6.40 -> 5.44.
+// Double division and square root that round correctly, as the operators do, but without branches:
+// an attempt holds 22 divisions, and each branch to a slow path ends the block that the compiler can
+// overlap, so a warp waited out one division after the other.
+//
+// They are Goldschmidt's iterations with Markstein's last step (P. Markstein, "Software Division and
+// Square Root Using Goldschmidt's Algorithms", 6th Conference on Real Numbers and Computers, 2004)
+// from PTX's approximate instructions, whose relative error of about 2^-20 is squared by each
+// iteration:
+//   1/b:      e = 1 - b y,  y <- y + y e (2^-40),  e <- e^2,  y <- y + y e (2^-80: an ulp of rounding)
+//             last step r = 1 - b y exactly,  y + y r
+//   a/b:      q = a y with y = 1/b rounded correctly,  last step r = a - b q exactly,  q + y r
+//   sqrt(x):  g = x y, h = y / 2;  twice r = 1/2 - g h,  g <- g + g r,  h <- h + h r  (g to sqrt(x), h to
+//             1 / (2 sqrt(x)); 2^-39, then an ulp);  last step d = x - g^2 exactly,  g + h d
+// The last step's multiply-add rounds an expression that is within 2^-51 ulp of the exact result, so only
+// results that close to a midpoint could round the other way; Markstein's theorem leaves one such
+// divisor, the significand of all ones.  They hold while operands, results and remainders are
+// normal numbers.  Outside that a ratio gives NaN or, for a quotient or remainder below the
+// normal range, a neighbour of the result: a zero, subnormal, infinite or NaN operand of ratio()
+// other than a zero numerator gives NaN, and so does a quotient that overflows.  inv() of zero,
+// of a subnormal and of an infinity is NaN too; its arguments here, r^2 + a^2 and r^4 + a^2 y^2,
+// take such values only where r itself is NaN already (r = r2 rsqrt(r2), 0 x inf).  The square
+// root keeps 0 and infinity.
 template <> struct Ops<double> {
     static __device__ __forceinline__ double rsq(double x) { return rsqrt(x); }
     static __device__ __forceinline__ double inv(double b) {
         double y;
         asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
         const double e = ::fma(-b, y, 1.0);
-        y = ::fma(y, ::fma(e, e, e), y);
+        y = ::fma(y, e, y);
+        y = ::fma(y, e * e, y);
         return ::fma(y, ::fma(-b, y, 1.0), y);
     }
     static __device__ __forceinline__ double ratio(double a, double b) {
@@ -70,10 +84,15 @@ template <> struct Ops<double> {
     static __device__ __forceinline__ double sqrt_rn(double x) {
         double y;
         asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-        const double e = ::fma(-x * y, y, 1.0);
-        y = ::fma(y * e, ::fma(0.375, e, 0.5), y);
-        const double s = x * y, c = ::fma(0.5 * y, ::fma(-s, s, x), s);
-        return x == 0.0 ? 0.0 : c;
+        double g = x * y, h = 0.5 * y;
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const double r = ::fma(-g, h, 0.5);
+            g = ::fma(g, r, g);
+            h = ::fma(h, r, h);
+        }
+        g = ::fma(h, ::fma(-g, g, x), g);
+        return x == 0.0 || x == __longlong_as_double(0x7ff0000000000000ll) ? x : g;
     }
     static __device__ __forceinline__ double fma(double a, double b, double c) { return ::fma(a, b, c); }
     static __device__ __forceinline__ double mul(double a, double b) { return __dmul_rn(a, b); }

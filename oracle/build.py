@@ -6,6 +6,8 @@
    its integrator knobs into the source, src/renderer/utils.rs:121-163).  Only built when the
    reference tree is present (the build container); the .so files travel with the repository
    snapshot to the GPU machine.
+3. oracle/libkt_probe.so  — device_probe.cu: single device functions of the product, built from its
+   headers with the flags of its kernels.
 
 The `#define` text is produced here independently of the product library, with Rust's
 `{:.10}` formatting of the f32 value (Python's exact decimal formatting of the same binary
@@ -25,6 +27,7 @@ ROOT = HERE.parent
 REF_DIR = Path(os.environ.get("KT_REFERENCE_DIR", "/root/reference"))
 REF_OUT = HERE / "_ref"
 ORACLE_LIB = HERE / "libkt_oracle.so"
+PROBE_LIB = HERE / "libkt_probe.so"
 REF_SCENES = ("c1", "c2", "t1", "t2")
 
 
@@ -43,6 +46,19 @@ def build_oracle(force: bool = False) -> Path:
           "-ffp-contract=off", "-fno-fast-math", str(src), "-o", str(tmp)])
     os.replace(tmp, ORACLE_LIB)
     return ORACLE_LIB
+
+
+def build_probe(force: bool = False) -> Path:
+    src, csrc = HERE / "device_probe.cu", ROOT / "kerrtrace_b200" / "csrc"
+    deps = [src, *csrc.glob("*.cuh"), *csrc.glob("*.h")]
+    if not force and PROBE_LIB.exists() and all(PROBE_LIB.stat().st_mtime >= p.stat().st_mtime for p in deps):
+        return PROBE_LIB
+    tmp = PROBE_LIB.with_suffix(".so.tmp")
+    _run([shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc", "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo",
+          "-O3", "-std=c++17", "-use_fast_math", "-shared", "-Xcompiler", "-fPIC", "-cudart", "static",
+          "-I", str(ROOT / "include"), "-I", str(csrc), str(src), "-o", str(tmp)])
+    os.replace(tmp, PROBE_LIB)
+    return PROBE_LIB
 
 
 def f32(x: float) -> float:
@@ -96,11 +112,13 @@ def build_reference(force: bool = False) -> list[Path]:
 
 def build(force: bool = False) -> None:
     build_oracle(force)
+    build_probe(force)
     build_reference(force)
 
 
 if __name__ == "__main__":
     build(force="--force" in sys.argv)
     print(ORACLE_LIB)
+    print(PROBE_LIB)
     for p in sorted(REF_OUT.glob("*.so")):
         print(p)

@@ -1,7 +1,7 @@
 """Shared fixtures.  Tests marked `gpu` need a CUDA device; everything else runs on CPU.
 
 The product library (kerrtrace_b200/libkerrtrace.so) and the checker libraries
-(oracle/libkt_oracle.so, oracle/_ref/*.so) are built by `python __graft_entry__.py` /
+(oracle/libkt_oracle.so, oracle/libkt_probe.so, oracle/_ref/*.so) are built by `python __graft_entry__.py` /
 `__graft_entry__.build()`; where nvcc is present and they are missing they are built here.
 """
 from __future__ import annotations
@@ -29,6 +29,8 @@ def _ensure_built():
         kbuild.build()
     if not obuild.ORACLE_LIB.exists():
         obuild.build_oracle()
+    if not obuild.PROBE_LIB.exists():
+        obuild.build_probe()
 
 
 _ensure_built()
