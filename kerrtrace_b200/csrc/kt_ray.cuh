@@ -474,9 +474,17 @@ __device__ __forceinline__ int ray_advance(RayRun<R>& ry, const Scene& sc, uint3
             e[c] = O::ratio(O::absr(h * (C::e1 * k1[c] + C::e3 * k3[c] + C::e4 * k4[c] + C::e5 * k5[c] +
                                          C::e6 * k6[c] + C::e7 * k7[c])), scale);
     }
-    R errv = O::maxr(O::maxr(O::maxr(e[0], e[1]), O::maxr(e[2], e[3])), O::maxr(e[4], e[5]));
+    R errv;
     if constexpr (std::is_same<R, double>::value) {
-        if (O::isnanr(errv)) {  // a zero tolerance or an infinite state: ratio() does not cover them
+        // Quotients of magnitudes, or NaN for an operand or a quotient that ratio() does not cover
+        // (an infinite component, a zero tolerance).  As integers they compare like the doubles,
+        // with every NaN on top; with one such component all six are divided by the operator.
+        unsigned long long top = 0;
+#pragma unroll
+        for (int c = 0; c < 6; ++c) top = max(top, (unsigned long long)__double_as_longlong(e[c]));
+        errv = __longlong_as_double((long long)top);
+        if ((unsigned)(top >> 32) >= 0x7ff00000u) {
+            errv = __longlong_as_double(0x7fffffffffffffffll);
 #pragma unroll
             for (int c = 0; c < 6; ++c) {
                 const R ec = O::absr(h * (C::e1 * k1[c] + C::e3 * k3[c] + C::e4 * k4[c] + C::e5 * k5[c] +
@@ -484,6 +492,8 @@ __device__ __forceinline__ int ray_advance(RayRun<R>& ry, const Scene& sc, uint3
                 errv = O::maxr(errv, ec / (ry.tol * O::maxr(O::absr(s[c]), R(1))));
             }
         }
+    } else {
+        errv = O::maxr(O::maxr(O::maxr(e[0], e[1]), O::maxr(e[2], e[3])), O::maxr(e[4], e[5]));
     }
     const bool ok = errv <= R(1);
     ry.h = h * lit<R>(0.9f, 0.9) * O::powr(errv, lit<R>(-0.2f, -0.2));

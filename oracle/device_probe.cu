@@ -57,9 +57,53 @@ __global__ void fp64_random_kernel(int op, uint64_t first, uint64_t per_thread, 
     if (bad) atomicAdd(differing, (unsigned long long)bad);
 }
 
+// One FP64 attempt of the stated physics from the state in[0..5] with k1 in[6..11], p_t, step size and
+// tolerance in[12..14]; out: the state after it, the next step size, the attempts spent on the
+// step (0 after a commit).
+__global__ void fp64_attempt_kernel(const __grid_constant__ ktd::Scene sc, const double* in, double* out,
+                                    uint32_t* err) {
+    ktd::RayRun<double> ry;
+    ktd::Tally tl;
+    tl.clear();
+    for (int c = 0; c < 6; ++c) {
+        ry.s[c] = in[c];
+        ry.k1[c] = in[6 + c];
+    }
+    ry.pt = in[12];
+    ry.kt = 0.0;
+    ry.h = in[13];
+    ry.tol = in[14];
+    ry.col[0] = ry.col[1] = ry.col[2] = 0.0;
+    ry.tau = 1.0;
+    ry.step = ry.attempt = 0;
+    ktd::ray_advance<double, 1, false, false>(ry, sc, err, tl, ktd::kRayGoing);
+    for (int c = 0; c < 6; ++c) out[c] = ry.s[c];
+    out[6] = ry.h;
+    out[7] = ry.attempt;
+}
+
 }  // namespace
 
 extern "C" {
+
+// mass, spin: of the hole; the disk, the sky and the escape radius are out of reach.
+int ktp_fp64_attempt(double mass, double spin, const double* in, double* out, uint32_t* err) {
+    ktd::Scene sc = {};
+    sc.M_d = mass;
+    sc.a_d = spin;
+    sc.aa_d = spin * spin;
+    sc.M = (float)mass;
+    sc.max_steps = sc.max_attempts = 10;
+    sc.escape_d = 1e300;
+    sc.disk_inner_d = 1e299;
+    sc.disk_outer_d = 1e300;
+    sc.base_tol_d = 1e-6;
+    sc.mode = 1;
+    sc.precision = 2;
+    fp64_attempt_kernel<<<1, 1>>>(sc, in, out, err);
+    const cudaError_t e = cudaGetLastError();
+    return (int)(e != cudaSuccess ? e : cudaDeviceSynchronize());
+}
 
 int ktp_fp64_op(int op, long long n, const double* a, const double* b, double* got, double* want) {
     if (n <= 0 || op < 0 || op > 2) return (int)cudaErrorInvalidValue;

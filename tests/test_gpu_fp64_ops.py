@@ -17,6 +17,7 @@ def probe():
     import oracle.build as obuild
     L = C.CDLL(str(obuild.PROBE_LIB))
     L.ktp_fp64_op.argtypes = [C.c_int, C.c_longlong] + 4 * [C.c_void_p]
+    L.ktp_fp64_attempt.argtypes = 2 * [C.c_double] + 3 * [C.c_void_p]
     L.ktp_fp64_random.argtypes = [C.c_int, C.c_ulonglong, C.c_int, C.c_int, C.c_int, C.c_void_p]
     return L
 
@@ -110,3 +111,27 @@ def test_ends_of_the_range(cuda, probe):
     b = [1.0, inf, 1.0, nan, 0.0, tiny, 0.0, 2.0 ** -1000, 1e-200, inf]
     got, want = run(cuda, probe, DIV, a, b)
     assert np.isnan(got).all(), (got, want)
+
+
+@pytest.mark.parametrize("component", [0, 1, 2])
+@pytest.mark.parametrize("h,accepted", [(1e-3, True), (1e14, False)])
+def test_a_step_with_one_error_component_out_of_range_is_rejected(cuda, probe, component, h, accepted):
+    """Straight motion along one axis (no mass), whose k1 is not its velocity: that component's error is
+    h x 71/57600, the other five are exactly 0.  Over scales of 5e-300 and more the quotient is 6e309
+    to 2.4e310 for h = 1e14, beyond the doubles: an infinite error, and a step that has to be tried
+    again.  The accepted step has h = 1e-3 and scales of 5 and more."""
+    x = np.zeros(15)
+    x[:3] = 20.0, 5.0, 7.0
+    x[3 + component] = 1.0
+    x[6 + component] = 2.0
+    x[12], x[13], x[14] = -1.0, h, 1.0 if accepted else 1e-300
+    d_in = cuda.tensor(x, device="cuda")
+    out = cuda.zeros(8, dtype=cuda.float64, device="cuda")
+    err = cuda.zeros(2, dtype=cuda.int32, device="cuda")
+    cuda.cuda.synchronize()
+    assert probe.ktp_fp64_attempt(0.0, 0.0, *[C.c_void_p(t.data_ptr()) for t in (d_in, out, err)]) == 0
+    got = out.cpu().numpy()
+    if accepted:
+        assert got[7] == 0 and got[component] != x[component]
+    else:
+        assert got[7] == 1 and np.array_equal(got[:6], x[:6]) and got[6] == 0.0
