@@ -1062,9 +1062,12 @@ static bool radius_fits(int R) {
     return (size_t)32 * ((kTPos + 2 * R) | 1) * 16 + (size_t)(2 * R + 2 + kTPos) * 4 <= kSmemLimit;
 }
 
+// Lets a kernel be launched with `bytes` of shared memory.  The attribute belongs to the function, not
+// to the launch, so it is always raised to the same limit: with the size of the call at hand, a
+// thread with a smaller radius could lower it between another's call and launch, which then failed.
 static cudaError_t set_smem(const void* fn, size_t bytes) {
     if (bytes <= 48 * 1024) return cudaSuccess;
-    return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemLimit);
 }
 
 // Radii above this (25583) are refused by every post entry point and have no tables.

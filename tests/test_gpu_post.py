@@ -231,3 +231,41 @@ def test_overlapped_launches_keep_stream_order(cuda, size, radius, graph):
     for q in range(2):
         for it in range(12):
             assert cuda.equal(got[q][it], want[(it + q) % 3]), (q, it)
+
+
+def test_post_passes_of_two_radii_from_two_threads(cuda):
+    """Two host threads whose contexts need different amounts of shared memory (radii 90 and 60, both
+    above the default limit) issue their passes at the same time: every call succeeds, and the images
+    are those of calls made one after the other."""
+    import threading
+    ctx, hdr, img, want, failed = [], [], [], [], []
+    for i, radius in enumerate((90.0, 60.0)):
+        cfg, _ = workloads.scene("t1")
+        cfg = workloads.scaled(cfg, 64, 40)
+        cfg.bloom_radius = radius
+        ctx.append(kt.Context(cfg))
+        hdr.append(_hdr_input(cuda, cfg, 21 + i))
+        img.append(cuda.zeros(64 * 40, dtype=cuda.int32, device="cuda"))
+        ctx[i].post_fused(hdr[i].data_ptr(), img[i].data_ptr())
+        cuda.cuda.synchronize()
+        want.append(img[i].clone())
+    streams = [cuda.cuda.Stream() for _ in ctx]
+    start = threading.Barrier(2)
+
+    def issue(i):
+        start.wait()
+        for _ in range(4000):
+            try:
+                ctx[i].post_fused(hdr[i].data_ptr(), img[i].data_ptr(), streams[i].cuda_stream)
+            except kt.KtError as e:
+                failed.append(str(e))
+
+    threads = [threading.Thread(target=issue, args=(i,)) for i in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    cuda.cuda.synchronize()
+    assert not failed, (len(failed), failed[0])
+    for i in range(2):
+        assert cuda.equal(img[i], want[i])
