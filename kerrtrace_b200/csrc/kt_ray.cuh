@@ -462,6 +462,9 @@ __device__ __forceinline__ int ray_advance(RayRun<R>& ry, const Scene& sc, uint3
                                 C::b6 * k6[c]);
         hamilton_rhs<R, EXACT>(nx, ry.pt, a, aa, M, k7);
     }
+    // an ended ray keeps its step size: grown or shrunk on, it would end in infinities and NaN, whose
+    // divisions, roots and powers take the slow paths of the double functions
+    if (TOGETHER && std::is_same<R, double>::value && state != kRayGoing) return state;
     // max-norm of the embedded error, per-component scale tol * max(|y_i|, 1)
     R e[6];
     if constexpr (PACKED) weigh<6>(e, {C::e1, C::e3, C::e4, C::e5, C::e6, C::e7}, {k1, k3, k4, k5, k6, k7});
