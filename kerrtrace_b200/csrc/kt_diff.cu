@@ -459,14 +459,13 @@ __device__ __forceinline__ R rk_a(int m, int j) {
 // patch of the frame, whose rays have more equal lengths than a row's 32 (512x512: FP32 437 -> 391
 // us with the host's tables, FP64 1.39 -> 1.14 ms).
 // RR: arithmetic type of the records (R, or float records replayed in double arithmetic).
-template <class R, bool REPLAY, class RR = R>
+template <class R, bool REPLAY, bool STRIPS, class RR = R>
 __global__ void __launch_bounds__(128, sizeof(R) == 8 ? 3 : 4) diff_forward_kernel(const Scene sc, const Camera cam, const CameraD camd,
                                                           const DiffRecRaw rec, float4* __restrict__ hdr,
                                                           double* __restrict__ hdr64, uint32_t* __restrict__ err,
                                                           uint32_t* __restrict__ flags) {
     int px, py;
-    tile_to_pixel(blockIdx.x * blockDim.x + threadIdx.x, sc.width, px, py);
-    if (px >= sc.width || py >= sc.height) return;
+    if (!frame_pixel(blockIdx.x * blockDim.x + threadIdx.x, sc.width, sc.height, STRIPS, px, py)) return;
     const unsigned p = (unsigned)py * (unsigned)sc.width + (unsigned)px;
     RayRun<R> ry;
     Tally tl;
@@ -951,22 +950,40 @@ __global__ void __launch_bounds__(128, BackMinBlocks<R>::v) diff_backward_kernel
 }
 
 // ---- launchers ----------------------------------------------------------------------------------
+template <bool STRIPS>
+static void forward_in_order(dim3 grid, const Scene& sc, const Camera& cam, const CameraD& camd, const DiffRecRaw& rec,
+                             bool replay, bool float_records, float4* hdr, double* hdr64, uint32_t* err, uint32_t* flags,
+                             cudaStream_t st) {
+    if (sc.precision == 2 && float_records)
+        diff_forward_kernel<double, true, STRIPS, float><<<grid, 128, 0, st>>>(sc, cam, camd, rec, hdr, hdr64, err, flags);
+    else if (sc.precision == 2 && replay)
+        diff_forward_kernel<double, true, STRIPS><<<grid, 128, 0, st>>>(sc, cam, camd, rec, hdr, hdr64, err, flags);
+    else if (sc.precision == 2)
+        diff_forward_kernel<double, false, STRIPS><<<grid, 128, 0, st>>>(sc, cam, camd, rec, hdr, hdr64, err, flags);
+    else if (replay)
+        diff_forward_kernel<float, true, STRIPS><<<grid, 128, 0, st>>>(sc, cam, camd, rec, hdr, hdr64, err, flags);
+    else
+        diff_forward_kernel<float, false, STRIPS><<<grid, 128, 0, st>>>(sc, cam, camd, rec, hdr, hdr64, err, flags);
+}
+
 cudaError_t launch_diff_forward(const Scene& sc, const Camera& cam, const CameraD& camd, const DiffRecRaw& rec,
                                 int replay, float4* hdr, double* hdr64, uint32_t* err, uint32_t* flags,
                                 cudaStream_t st, bool float_records) {
     const unsigned n = (unsigned)sc.width * (unsigned)sc.height;
     if (n == 0) return cudaSuccess;
-    const dim3 grid(unit_count(sc.width, sc.height, 1, false) / 4);  // 128 pixels of a 16x16 tile each
-    if (sc.precision == 2 && float_records) {
-        if (!replay) return cudaErrorInvalidValue;
-        diff_forward_kernel<double, true, float><<<grid, 128, 0, st>>>(sc, cam, camd, rec, hdr, hdr64, err, flags);
-    } else if (sc.precision == 2) {
-        if (replay) diff_forward_kernel<double, true><<<grid, 128, 0, st>>>(sc, cam, camd, rec, hdr, hdr64, err, flags);
-        else diff_forward_kernel<double, false><<<grid, 128, 0, st>>>(sc, cam, camd, rec, hdr, hdr64, err, flags);
-    } else {
-        if (replay) diff_forward_kernel<float, true><<<grid, 128, 0, st>>>(sc, cam, camd, rec, hdr, hdr64, err, flags);
-        else diff_forward_kernel<float, false><<<grid, 128, 0, st>>>(sc, cam, camd, rec, hdr, hdr64, err, flags);
+    bool strips = false;
+    if (patches_idle(sc.width, sc.height)) {
+        int dev = 0, sms = 0;
+        cudaError_t e = cudaGetDevice(&dev);
+        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        if (e != cudaSuccess) return e;
+        strips = take_strips(sc.width, sc.height, unit_count(sc.width, sc.height, 1, false, false),
+                             (unsigned)sms * (sc.precision == 2 ? 12u : 16u));
     }
+    const dim3 grid((index_count(sc.width, sc.height, strips) + 127) / 128);
+    if (sc.precision == 2 && float_records && !replay) return cudaErrorInvalidValue;
+    if (strips) forward_in_order<true>(grid, sc, cam, camd, rec, replay, float_records, hdr, hdr64, err, flags, st);
+    else forward_in_order<false>(grid, sc, cam, camd, rec, replay, float_records, hdr, hdr64, err, flags, st);
     return cudaGetLastError();
 }
 

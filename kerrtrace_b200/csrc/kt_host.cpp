@@ -1197,6 +1197,7 @@ void kt_renderer_destroy(kt_renderer* r) { destroy_renderer(r); }
 // =========================================================================================
 struct kt_batch {
     int device = 0;
+    int sms = 0;
     std::vector<kt_context*> ctx;
     std::vector<kt_job> jobs;
     ktd::BatchTable* table = nullptr;
@@ -1218,7 +1219,11 @@ void batch_drop_graph(kt_batch* b) {
 }
 void batch_layout(kt_batch* b) {
     int tiles = 0;
-    unsigned units = 0;
+    unsigned units = 0, patch_units = 0;
+    for (int j = 0; j < b->table->n; ++j)
+        patch_units += ktd::unit_count(b->table->job[j].sc.width, b->table->job[j].sc.height, 1, false, false);
+    // warps that the GPU holds of the kernel's default shape (launch_batch_persistent)
+    const unsigned warps = (unsigned)b->sms * (b->table->job[0].sc.precision == KT_PREC_FP64 ? 8u : 16u);
     for (int j = 0; j < b->table->n; ++j) {
         ktd::BatchJob& e = b->table->job[j];
         e.tiles_x = (e.sc.width + b->bx - 1) / b->bx;
@@ -1226,7 +1231,8 @@ void batch_layout(kt_batch* b) {
         e.tile_begin = tiles;
         tiles += e.tiles_x * tiles_y;
         e.unit_begin = units;
-        units += ktd::unit_count(e.sc.width, e.sc.height, 1, false);
+        e.strips = ktd::take_strips(e.sc.width, e.sc.height, patch_units, warps) ? 1 : 0;
+        units += ktd::unit_count(e.sc.width, e.sc.height, 1, false, e.strips != 0);
     }
     b->table->total_tiles = tiles;
     b->table->total_units = units;
@@ -1285,15 +1291,16 @@ kt_status kt_batch_create(const kt_job* jobs, uint32_t n, int device, kt_batch**
         e.hdr = reinterpret_cast<float4*>(jobs[j].hdr_out);
         e.err = jobs[j].err_word;
     }
-    batch_layout(b);
     {
         DeviceGuard g(device);
-        const cudaError_t e = cudaMalloc(&b->counter, sizeof(unsigned));
+        cudaError_t e = cudaDeviceGetAttribute(&b->sms, cudaDevAttrMultiProcessorCount, device);
+        if (e == cudaSuccess) e = cudaMalloc(&b->counter, sizeof(unsigned));
         if (e != cudaSuccess) {
             batch_free(b);
             return cuda_fail(e, "allocate the unit counter");
         }
     }
+    batch_layout(b);
     *out = b;
     return KT_OK;
 }

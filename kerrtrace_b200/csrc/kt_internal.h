@@ -48,13 +48,67 @@ cudaError_t launch_trace(const Scene& sc, const Camera& cam, int schedule, float
                          uint32_t* err, unsigned* queue, unsigned long long* ctr, float4* aux,
                          const Tuning& tn, int bx, int by, unsigned* order, cudaStream_t stream);
 
-// Units of 32 / S pixels that cover a frame: whole tiles, or exactly its pixels when they come
+// ---- order in which the units take the pixels of a frame ---------------------------------------
+// A unit is a run of 32 / S indices; frame_pixel turns an index into a pixel.  Patches: 16x16 tiles in
+// raster order, Morton order inside a tile, so that an aligned run of 32, 16, 8, ... indices is a
+// patch of 8x4, 4x4, 4x2, ... pixels.  The indices cover whole tiles: some name no pixel.  Strips: the
+// frame cut into strips of about 8 columns, each numbered row by row, one after the other: exactly
+// one index per pixel, and a run of 32 is about as square.
+//
+// In frames with short sides the patches leave lanes idle: 28 of 32 at one column, 24 at one row, a
+// third at 17 columns.  A launch that fills the GPU pays for them, so it takes strips where less than
+// 15 of 16 lanes of the patches with a pixel have one (below about 110 columns or 60 rows).
+// Patches -> strips, FP32: 64 persistent renders of 1x8192 5.42 -> 0.77 ms, of 17x4096 8.17 -> 5.74; a
+// frame of 1x32768 374 -> 103 us; eight views of it 2.64 -> 0.41 ms; recording forward of 9x32768 609 ->
+// 388 us.
+// A launch whose patches all start at once lasts as long as its longest warp, and a warp with idle
+// lanes is shorter: it keeps the patches.
+// (patches and strips: frame of 1x1080 80 and 97 us, recording forward in FP64 of 300x33 334 and 385.)
+// The kernels are instances for one order or the other: with both in one, the large launches of the
+// mixed trace and of the views call were 0.5% slower.  Launch shapes of the wavefront schedule other
+// than the default (blocks per SM, counting) keep the patches.
+__host__ __device__ inline bool patches_idle(int W, int H) {
+    const unsigned w = ((unsigned)W + 7u) & ~7u, h = ((unsigned)H + 3u) & ~3u;
+    return 16ull * ((unsigned)W * (unsigned)H) < 15ull * (w * h);
+}
+// Indices of a frame.
+__host__ __device__ inline unsigned index_count(int W, int H, bool strips) {
+    return strips ? (unsigned)W * (unsigned)H : ((unsigned)(W + 15) >> 4) * ((unsigned)(H + 15) >> 4) * 256u;
+}
+// The pixel of an index; false when it has none (outside the frame, or beyond the last index).
+__host__ __device__ inline bool frame_pixel(unsigned idx, int W, int H, bool strips, int& px, int& py) {
+    if (strips) {
+        // n strips, strip i from column i W / n on: i W / n H indices lie before it, so idx / H is one
+        // of the columns of idx's strip
+        const unsigned n = W < 12 ? 1u : ((unsigned)W + 4u) >> 3;
+        const unsigned column = idx / (unsigned)H;
+        const unsigned strip = ((column + 1u) * n - 1u) / (unsigned)W;
+        const unsigned x0 = strip * (unsigned)W / n, x1 = (strip + 1u) * (unsigned)W / n;
+        const unsigned at = idx - x0 * (unsigned)H, w = x1 - x0;
+        py = (int)(at / w);
+        px = (int)(x0 + at - (unsigned)py * w);
+        return column < (unsigned)W;
+    }
+    const unsigned tiles_x = ((unsigned)W + 15u) >> 4;
+    const unsigned tile = idx >> 8, m = idx & 255u;
+    const unsigned ty = tile / tiles_x, tx = tile - ty * tiles_x;
+    const unsigned x = (m & 1u) | (m >> 1 & 2u) | (m >> 2 & 4u) | (m >> 3 & 8u);
+    const unsigned y = (m >> 1 & 1u) | (m >> 2 & 2u) | (m >> 3 & 4u) | (m >> 4 & 8u);
+    px = (int)(tx * 16u + x);
+    py = (int)(ty * 16u + y);
+    return px < W && py < H;
+}
+// Units of 32 / S pixels that cover a frame: all its indices, or exactly its pixels when they come
 // from a pixel-order buffer.
-__host__ __device__ inline unsigned unit_count(int W, int H, int S, bool ordered) {
+__host__ __device__ inline unsigned unit_count(int W, int H, int S, bool ordered, bool strips) {
     const unsigned P = 32u / (unsigned)S;
-    const unsigned n = ordered ? (unsigned)W * (unsigned)H
-                               : ((unsigned)(W + 15) >> 4) * ((unsigned)(H + 15) >> 4) * 256u;
+    const unsigned n = ordered ? (unsigned)W * (unsigned)H : index_count(W, H, strips);
     return (n + P - 1u) / P;
+}
+// The rule above: whether a frame takes strips in a launch of `patch_units` units, counted in patches
+// over all its frames, on a GPU that holds `warps` of the kernel's warps.
+inline bool take_strips(int W, int H, unsigned patch_units, unsigned warps) {
+    return patch_units > warps && patches_idle(W, H);
 }
 
 #ifdef __CUDACC__
@@ -104,6 +158,7 @@ struct BatchJob {
     int tiles_x;
     int tile_begin;
     unsigned unit_begin;  // persistent launch: first 32-pixel unit of this job
+    int strips;           // and its pixel order
 };
 struct BatchTable {
     BatchJob job[kBatchMaxJobs];

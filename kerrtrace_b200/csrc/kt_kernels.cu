@@ -252,7 +252,7 @@ __global__ void __launch_bounds__(MAXT, MINB)
 // 960x540 FP64 5.67 -> 2.42, 1024^2 mixed 2.64 -> 1.09, two frames of 2100x900 at 4 samples 16.0 -> 7.16;
 // 96x64 at 2 samples 0.277 -> 0.080, where a pixel's samples used to run one after the other on one lane; with
 // frozen rays kept to the end (a switch for timing) 183 -> 187.
-template <class R, int MODE, bool COUNT, int MINB, bool TOGETHER>
+template <class R, int MODE, bool COUNT, int MINB, bool TOGETHER, bool STRIPS>
 __global__ void __launch_bounds__(kWavefrontBlock, MINB)
     trace_wavefront_kernel(const __grid_constant__ Scene sc, const Camera cam, float4* __restrict__ hdr,
                            uint32_t* __restrict__ err, unsigned* __restrict__ queue,
@@ -263,7 +263,7 @@ __global__ void __launch_bounds__(kWavefrontBlock, MINB)
     const int slot = lane / S, sub = lane - slot * S;
     const unsigned P = 32u / (unsigned)S;
     const unsigned n_px = (unsigned)sc.width * (unsigned)sc.height;
-    const unsigned units = unit_count(sc.width, sc.height, S, order != nullptr);
+    const unsigned units = unit_count(sc.width, sc.height, S, order != nullptr, STRIPS);
     const unsigned n_hot = order ? order[0] : 0u;
     const unsigned n_warps = gridDim.x * (kWavefrontBlock / 32);
     Tally total;
@@ -278,8 +278,7 @@ __global__ void __launch_bounds__(kWavefrontBlock, MINB)
             valid = valid && idx < n_px;
             if (valid) ordered_pixel(idx, n_px, order, n_hot, sc.width, px, py);
         } else {
-            tile_to_pixel(idx, sc.width, px, py);
-            valid = valid && px < sc.width && py < sc.height;
+            valid = valid && frame_pixel(idx, sc.width, sc.height, STRIPS, px, py);
         }
         float acc[3] = {0.0f, 0.0f, 0.0f};
         for (int s0 = 0; s0 < sc.spp; s0 += S) {
@@ -362,8 +361,13 @@ static cudaError_t launch_wave_minb(const Scene& sc, const Camera& cam, float4* 
     if (e != cudaSuccess) return e;
     constexpr unsigned kWarps = kWavefrontBlock / 32;
     const int S = samples_in_parallel(sc.spp);
-    const unsigned units = unit_count(sc.width, sc.height, S, order != nullptr);
-    const unsigned blocks = (units + kWarps - 1) / kWarps, resident = (unsigned)(sms * MINB);
+    const unsigned resident = (unsigned)(sms * MINB);
+    const bool ordered = order != nullptr;
+    constexpr bool kDefaultShape = !COUNT && MINB == WaveDefaults<R>::minb;  // the others keep the patches
+    const bool strips = kDefaultShape && !ordered &&
+                        take_strips(sc.width, sc.height, unit_count(sc.width, sc.height, S, false, false), resident * kWarps);
+    const unsigned units = unit_count(sc.width, sc.height, S, ordered, strips);
+    const unsigned blocks = (units + kWarps - 1) / kWarps;
     // Stated physics in FP32 and FP64: a block per four units, not only the resident ones.  The
     // hardware's block scheduler then hands out the units and the warps of a block start
     // together, at the same place of a loop body (30 KB in FP64) that outgrows the nearer instruction
@@ -381,18 +385,23 @@ static cudaError_t launch_wave_minb(const Scene& sc, const Camera& cam, float4* 
     // that keeps its lanes in step issues fewer instructions for them (96x64 x 2 samples 78.3 -> 72.2
     // us, 256x256 at tolerance 1e-8 23.9 -> 23.3 ms).  With more units the vote and the register
     // moves around it cost more than they save (1920x1080 2.21 -> 2.37 ms).
-    if constexpr (!COUNT && MINB == WaveDefaults<R>::minb) {
+    if constexpr (kDefaultShape) {
+        if (strips) {
+            trace_wavefront_kernel<R, MODE, COUNT, MINB, false, true>
+                <<<grid, kWavefrontBlock, 0, st>>>(sc, cam, hdr, err, queue, ctr, aux, S, order);
+            return cudaGetLastError();
+        }
         if (units <= resident * kWarps) {
             if (order) {
-                trace_wavefront_kernel<R, MODE, COUNT, MINB, true>
+                trace_wavefront_kernel<R, MODE, COUNT, MINB, true, false>
                     <<<grid, kWavefrontBlock, 0, st>>>(sc, cam, hdr, err, queue, ctr, aux, S, order);
                 return cudaGetLastError();
             }
-            return launch_early(trace_wavefront_kernel<R, MODE, COUNT, MINB, true>, dim3(grid), kWavefrontBlock, 0, st, sc,
-                                cam, hdr, err, queue, ctr, aux, S, order);
+            return launch_early(trace_wavefront_kernel<R, MODE, COUNT, MINB, true, false>, dim3(grid), kWavefrontBlock, 0,
+                                st, sc, cam, hdr, err, queue, ctr, aux, S, order);
         }
     }
-    trace_wavefront_kernel<R, MODE, COUNT, MINB, false>
+    trace_wavefront_kernel<R, MODE, COUNT, MINB, false, false>
         <<<grid, kWavefrontBlock, 0, st>>>(sc, cam, hdr, err, queue, ctr, aux, S, order);
     return cudaGetLastError();
 }
@@ -481,7 +490,7 @@ cudaError_t launch_batch(const BatchTable& bt, int bx, int by, cudaStream_t st) 
     return launch_batch_typed<float, 0>(bt, bx, by, st);
 }
 
-// Persistent batched trace.  Every job is cut into units of 32 pixels (tile_to_pixel's order, so a
+// Persistent batched trace.  Every job is cut into units of 32 pixels (frame_pixel's order, so a
 // unit is an 8x4 patch of one frame); job j owns units [unit_begin, unit_begin of j + 1).  A
 // warp's first unit is its own index in the grid, the others come from a single device counter
 // over all jobs, so the 32 rays of a warp always share one scene and its parameters stay uniform
@@ -508,8 +517,7 @@ __global__ void __launch_bounds__(kWavefrontBlock, MINB)
         const BatchJob& jb = bt.job[lo];
         const Scene& sc = jb.sc;
         int px, py;
-        tile_to_pixel((u - jb.unit_begin) * 32u + (unsigned)lane, sc.width, px, py);
-        const bool valid = px < sc.width && py < sc.height;
+        const bool valid = frame_pixel((u - jb.unit_begin) * 32u + (unsigned)lane, sc.width, sc.height, jb.strips != 0, px, py);
         float acc[3] = {0.0f, 0.0f, 0.0f};
         Tally total;
         total.clear();

@@ -46,7 +46,7 @@ constexpr int kNoallocBlock = 128;
 // in the grid, the others come from one counter over all views.  (Refilling single lanes, as an
 // earlier form did, ran the ray set-up for one lane of 32: 8 views of 480x270 1.78 ms, now 1.22; at
 // 4 samples 8.55, now 4.59; 12 views of 64x36 at 2 samples 418 us, now 162.)
-template <bool TOGETHER>
+template <bool TOGETHER, bool STRIPS>
 __global__ void __launch_bounds__(kNoallocBlock, 4)
     trace_views_noalloc_kernel(const __grid_constant__ Scene sc, const __grid_constant__ NoallocViews views,
                                float4* __restrict__ hdr, uint32_t* __restrict__ err, unsigned* __restrict__ queue,
@@ -55,15 +55,16 @@ __global__ void __launch_bounds__(kNoallocBlock, 4)
     const int lane = threadIdx.x & 31;
     const int slot = lane / S, sub = lane - slot * S;
     const unsigned P = 32u / (unsigned)S;
-    const unsigned per_view = unit_count(sc.width, sc.height, S, false), units = per_view * (unsigned)views.n;
+    const unsigned per_view = unit_count(sc.width, sc.height, S, false, STRIPS);
+    const unsigned units = per_view * (unsigned)views.n;
     const unsigned n_warps = gridDim.x * (kNoallocBlock / 32);
     const size_t n_px = (size_t)sc.width * sc.height;
     for (unsigned u = blockIdx.x * (kNoallocBlock / 32) + (threadIdx.x >> 5); u < units;) {
         const unsigned view = u / per_view;
         const Camera& cam = views.cam[view];
-        int px, py;
-        tile_to_pixel((u - view * per_view) * P + (unsigned)slot, sc.width, px, py);
-        const bool valid = (unsigned)slot < P && px < sc.width && py < sc.height;
+        int px = 0, py = 0;
+        const bool valid = (unsigned)slot < P && frame_pixel((u - view * per_view) * P + (unsigned)slot, sc.width,
+                                                             sc.height, STRIPS, px, py);
         float acc[3] = {0.0f, 0.0f, 0.0f};
         for (int s0 = 0; s0 < sc.spp; s0 += S) {
             const int smp = s0 + sub;
@@ -166,17 +167,23 @@ extern "C" kt_status kt_trace_noalloc(const kt_config* cfg, const kt_camera* cam
     constexpr unsigned kWarps = kNoallocBlock / 32;
     int S = samples_in_parallel(sc.spp);
     // the unit counter is 32 bits wide (whole tiles of a large frame, up to a unit per pixel)
-    if ((uint64_t)unit_count(sc.width, sc.height, S, false) * n_views > 0x7fffffffu) S = 1;
-    const unsigned units = unit_count(sc.width, sc.height, S, false) * n_views;
-    const unsigned blocks = (units + kWarps - 1) / kWarps, resident = (unsigned)sms * 4u;
+    if ((uint64_t)unit_count(sc.width, sc.height, S, false, false) * n_views > 0x7fffffffu) S = 1;
+    const unsigned resident = (unsigned)sms * 4u;
+    const bool strips = take_strips(sc.width, sc.height, unit_count(sc.width, sc.height, S, false, false) * n_views,
+                                    resident * kWarps);
+    const unsigned units = unit_count(sc.width, sc.height, S, false, strips) * n_views;
+    const unsigned blocks = (units + kWarps - 1) / kWarps;
     const unsigned grid = blocks < resident ? blocks : resident;
     float4* hdr = reinterpret_cast<float4*>(hdr_out);
-    if (units <= grid * kWarps) {  // one unit per warp: lanes in step, as in launch_wave_minb
-        trace_views_noalloc_kernel<true><<<grid, kNoallocBlock, 0, s>>>(sc, views, hdr, err_words, queue, S);
+    if (units <= grid * kWarps && !strips) {  // one unit per warp: lanes in step, as in launch_wave_minb
+        trace_views_noalloc_kernel<true, false><<<grid, kNoallocBlock, 0, s>>>(sc, views, hdr, err_words, queue, S);
     } else {
         if ((e = cudaMemsetAsync(queue, 0, sizeof(unsigned), s)) != cudaSuccess)
             return set_error(KT_ERR_CUDA, cudaGetErrorString(e));
-        trace_views_noalloc_kernel<false><<<grid, kNoallocBlock, 0, s>>>(sc, views, hdr, err_words, queue, S);
+        if (strips)
+            trace_views_noalloc_kernel<false, true><<<grid, kNoallocBlock, 0, s>>>(sc, views, hdr, err_words, queue, S);
+        else
+            trace_views_noalloc_kernel<false, false><<<grid, kNoallocBlock, 0, s>>>(sc, views, hdr, err_words, queue, S);
     }
     if ((e = cudaGetLastError()) != cudaSuccess) return set_error(KT_ERR_CUDA, cudaGetErrorString(e));
     return KT_OK;

@@ -76,18 +76,6 @@ struct Tally {
     }
 };
 
-// Unit index -> pixel in 16x16 tiles (raster order), Morton order inside a tile: an aligned run of
-// 32, 16, 8, ... indices is a patch of 8x4, 4x4, 4x2, ... pixels.  The index space covers whole
-// tiles, so at the right and bottom border it names pixels outside the frame.
-__device__ __forceinline__ void tile_to_pixel(unsigned idx, int W, int& px, int& py) {
-    const unsigned tiles_x = ((unsigned)W + 15u) >> 4;
-    const unsigned tile = idx >> 8, m = idx & 255u;
-    const unsigned ty = tile / tiles_x, tx = tile - ty * tiles_x;
-    const unsigned x = (m & 1u) | (m >> 1 & 2u) | (m >> 2 & 4u) | (m >> 3 & 8u);
-    const unsigned y = (m >> 1 & 1u) | (m >> 2 & 2u) | (m >> 3 & 4u) | (m >> 4 & 8u);
-    px = (int)(tx * 16u + x);
-    py = (int)(ty * 16u + y);
-}
 // Lanes per pixel of the persistent tracer: the largest S <= min(spp, 32) that keeps 15 of 16
 // lanes busy over the pixel's samples (S lanes take spp samples in ceil(spp / S) rounds, and
 // 32 mod S lanes have no pixel).

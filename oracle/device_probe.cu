@@ -2,11 +2,13 @@
 // INFRASTRUCTURE ONLY: built from the product's headers with the flags of its kernels, so that
 // functions which no entry point exposes by themselves can be compared with CUDA's own.
 //
-// Every launch is one thread per operand, in bounds by construction; the C functions take device
-// pointers, run on the legacy stream and return the CUDA status after a synchronisation.
+// Every launch is one thread per operand, in bounds by construction; the C functions with launches
+// take device pointers, run on the legacy stream and return the CUDA status after a
+// synchronisation.  The unit order is host code and needs no device.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "kt_internal.h"
 #include "kt_ray.cuh"
 
 namespace {
@@ -119,6 +121,21 @@ int ktp_fp64_random(int op, unsigned long long first, int blocks, int per_thread
     fp64_random_kernel<<<blocks, 128>>>(op, first, (uint64_t)per_thread, max_exponent, differing);
     const cudaError_t e = cudaGetLastError();
     return (int)(e != cudaSuccess ? e : cudaDeviceSynchronize());
+}
+
+// The units of a frame at S lanes per pixel, the pixels of its first n indices (-1: none), and whether
+// it takes strips in a launch of that many patch units.
+unsigned ktp_unit_count(int width, int height, int S, int strips) {
+    return ktd::unit_count(width, height, S, false, strips != 0);
+}
+void ktp_frame_pixels(int width, int height, int strips, long long n, int* pixel) {
+    for (long long i = 0; i < n; ++i) {
+        int px = -1, py = -1;
+        pixel[i] = ktd::frame_pixel((unsigned)i, width, height, strips != 0, px, py) ? py * width + px : -1;
+    }
+}
+int ktp_take_strips(int width, int height, unsigned patch_units, unsigned warps) {
+    return ktd::take_strips(width, height, patch_units, warps) ? 1 : 0;
 }
 
 }  // extern "C"
