@@ -8,12 +8,13 @@
 //              shape; 128-thread blocks may ask for more resident blocks per SM, which caps
 //              registers per thread)
 //   wavefront  persistent blocks of 128 threads; warps take units of 32 rays from a device
-//              work counter (resident blocks per SM; the refill values of the list run the
-//              same kernel)
+//              work counter (resident blocks per SM)
 // each in tile order and in long-rays-first order.  Every candidate must reproduce the first
 // candidate's image bit for bit (they run the same per-ray arithmetic; a device kernel counts
 // differing pixels).  Each is timed with CUDA events on the caller's stream, `reps` launches
 // after one warm-up launch, and scored by the median; the fastest identical one is installed.
+// refill_min has no effect on any launch: a candidate that differs from an earlier one in it alone is
+// not run, and its row repeats the earlier one's figures (so the earlier one wins).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -48,7 +49,7 @@ kt_tuning make(int schedule, int bx, int by, int bps, int refill, int order, int
 std::vector<kt_tuning> default_candidates(int precision, int mode, int keep_frozen) {
     static const int kPlain[][2] = {{16, 16}, {32, 8}, {8, 8}, {16, 8}, {32, 4}, {8, 16}};
     static const int kPlain128[][2] = {{16, 8}, {8, 16}, {32, 4}};
-    static const int kRefill[] = {1, 4, 8, 16};
+    static const int kRefill[] = {1, 4, 8, 16};  // rows that callers look up; only the first is run
     std::vector<kt_tuning> out;
     for (int order : {KT_ORDER_TILES, KT_ORDER_LONG_FIRST}) {
         for (const auto& b : kPlain) out.push_back(make(KT_SCHED_PLAIN, b[0], b[1], 4, 1, order, keep_frozen));
@@ -63,6 +64,12 @@ std::vector<kt_tuning> default_candidates(int precision, int mode, int keep_froz
             for (int r : kRefill) out.push_back(make(KT_SCHED_WAVEFRONT, 0, 0, b, r, order, keep_frozen));
     }
     return out;
+}
+
+// Whether two tunings make the same launch.
+bool same_launch(const kt_tuning& a, const kt_tuning& b) {
+    return a.schedule == b.schedule && a.block_x == b.block_x && a.block_y == b.block_y &&
+           a.blocks_per_sm == b.blocks_per_sm && a.order == b.order && a.keep_frozen == b.keep_frozen;
 }
 
 // Device buffers of one tuning run, released on every path.
@@ -137,6 +144,15 @@ extern "C" kt_status kt_context_autotune(kt_context* ctx, void* stream, const kt
     rows.reserve(cands.size());
     for (size_t i = 0; i < cands.size(); ++i) {
         if ((st = kt_context_set_tuning(ctx, &cands[i])) != KT_OK) return st;
+        const auto earlier = std::find_if(rows.begin(), rows.end(), [&](const kt_tune_entry& r) {
+            return same_launch(r.tuning, cands[i]);
+        });
+        if (earlier != rows.end()) {
+            kt_tune_entry row = *earlier;
+            row.tuning = cands[i];
+            rows.push_back(row);
+            continue;
+        }
         if ((e = cudaMemsetAsync(sc.err, 0, 2 * sizeof(uint32_t), s)) != cudaSuccess) return tune_fail(e, "clear error word");
         if ((st = kt_trace(ctx, stream, cam, KT_SCHED_AUTO, sc.hdr, sc.err)) != KT_OK) return st;
         unsigned long long diff = 0;

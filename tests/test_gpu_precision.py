@@ -84,6 +84,25 @@ def test_autotune_picks_an_identical_and_fastest_shape(cuda):
         ctx.set_tuning(schedule=kt.SCHED_WAVEFRONT, blocks_per_sm=9)
 
 
+def test_autotune_runs_each_launch_once(cuda):
+    """refill_min has no effect: rows that differ in it alone repeat one measurement, the first of them
+    wins, and a value out of its range is refused as before."""
+    cfg, cam = workloads.scene("c2")
+    ctx = kt.Context(workloads.scaled(cfg, 160, 90))
+    res = autotune.autotune(ctx, cam, reps=2)
+    groups = {}
+    for ms, c, ok in res.table:
+        groups.setdefault(tuple(v for k, v in sorted(c.items()) if k != "refill_min"), []).append((ms, ok))
+    assert len(res.table) == 56 and len(groups) == 32
+    assert all(len(set(rows)) == 1 for rows in groups.values()), [r for r in groups.values() if len(set(r)) > 1]
+    assert ctx.tuning().refill_min == 1
+    bad = [dict(schedule=kt.SCHED_WAVEFRONT, block_x=0, block_y=0, blocks_per_sm=4, refill_min=r, order=0,
+                keep_frozen=0) for r in (1, 33)]
+    with pytest.raises(kt.KtError):
+        autotune.autotune(ctx, cam, reps=1, cands=bad)
+    ctx.close()
+
+
 def test_c3_draws_against_f64_oracle_on_strided_pixels(cuda, orc):
     """The 4096^2 mixed-precision ablation scenes (8 draws of spin and inclination, stated
     physics, tolerance 1e-6): the FP64, FP32 and mixed GPU images against the f64 oracle on every
