@@ -58,9 +58,12 @@ typedef enum kt_mode { KT_MODE_REF = 0, KT_MODE_SPEC = 1 } kt_mode;
 typedef enum kt_precision { KT_PREC_FP32 = 0, KT_PREC_MIXED = 1, KT_PREC_FP64 = 2 } kt_precision;
 
 /* Scheduling of the trace kernel.  All schedules produce the same image bits at one sample per pixel.
- * With more, the reference-semantics wavefront kernel rounds one product of a later sample's ray
- * start the other way round, so a few rays of some cameras differ from the plain schedule by an ulp
- * there. */
+ * With more, the wavefront schedule of a single frame (kt_trace and the renderer, in every mode and
+ * precision) and kt_trace_noalloc round one product in the ray start of the second and later samples
+ * the other way round: at some camera positions a few percent of the pixels then differ from the plain
+ * schedule's in the last places, or by a sky line.  Progressive sampling and both schedules of a batch
+ * have the plain schedule's bits at any number of samples.  The autotuner compares with its first
+ * candidate, so at such a camera it keeps plain shapes only. */
 typedef enum kt_schedule {
     KT_SCHED_PLAIN = 0,     /* one thread per pixel on a 2D grid of block_dim tiles (kernel.cu:88) */
     KT_SCHED_WAVEFRONT = 1, /* warps take units of 32 rays: a persistent kernel whose warps draw further units
@@ -258,8 +261,8 @@ kt_status kt_trace_counted(kt_context* ctx, void* stream, const kt_camera* cam,
  * the reference's jitter keys (pixel index << 32 | sample index), continues the running sum of
  * the raw sample colours in accum (dev float[4*W*H]: rgb = sum, w = samples so far; read when
  * first_sample > 0, written every call) and writes hdr_out = sum x (float)(exposure x (1.0f /
- * samples so far)).  After samples 0..N-1, in any split, hdr_out is bit for bit the kt_trace
- * image of the same scene at spp = N.  Samples are always jittered (also in stated physics,
+ * samples so far)).  After samples 0..N-1, in any split, hdr_out is bit for bit the plain
+ * schedule's kt_trace image of the same scene at spp = N.  Samples are always jittered (also in stated physics,
  * whose spp = 1 trace uses the pixel centre).  Plain schedule, stream-ordered. */
 kt_status kt_trace_progressive(kt_context* ctx, void* stream, const kt_camera* cam, uint32_t first_sample,
                                uint32_t n_samples, float* accum, float* hdr_out, uint32_t* err_word);

@@ -116,9 +116,10 @@ __device__ __forceinline__ void pixel_ray(int px, int py, int sample, const Scen
 //
 // N_z = r z + a x is a sum of two products, so it has two fused forms, which differ in the last
 // place for some camera positions.  The reference kernel's, and the plain schedule's, is
-// fma(a, x, r z).  The persistent schedules start the second and later samples of a pixel with
-// fma(r, z, a x) (later_sample): an ulp in l_z, which moves a sky line by a pixel here and there.
-// Both are written out so that each schedule keeps its own image bits.
+// fma(a, x, r z).  The persistent trace of a single frame (every mode and precision) and of the views
+// call start the second and later samples of a pixel with fma(r, z, a x) (later_sample): an ulp in
+// l_z, which moves a sky line by a pixel here and there.  The batch and progressive sampling do not.
+// Both forms are written out so that each keeps its own image bits.
 template <class R>
 __device__ __forceinline__ bool ray_start(RayRun<R>& ry, const Camera& cam, const float dir[3],
                                           const Scene& sc, bool later_sample = false) {

@@ -112,3 +112,32 @@ def test_recording_forward_in_strips(cuda, size):
     ctx.close()
     assert np.array_equal(hdr.cpu().numpy().view(np.uint32), want.view(np.uint32))
     d.close()
+
+
+@pytest.mark.parametrize("mode,prec", KINDS)
+@pytest.mark.parametrize("spin,radius,inclination", [(0.84, 60.0, 20.0), (-0.23, 30.0, 80.0), (-0.01, 120.0, 55.0)])
+def test_schedules_agree_as_documented(cuda, mode, prec, spin, radius, inclination):
+    """What kt_schedule promises over cameras, spins and kinds: one sample, every schedule of a frame and of a
+    batch has the plain image's bits; three samples, both schedules of a batch have them."""
+    base, _ = workloads.scene("c2")
+    cfg = workloads.scaled(base, 96, 54)
+    cfg.spin, cfg.mode, cfg.precision = spin, mode, prec
+    cam = kt.orbit_camera(radius, inclination, 30.0, azimuth_deg=100.0)
+    n = cfg.width * cfg.height
+    for spp in (1, 3):
+        cfg.spp = spp
+        want, _, _, ctx = run_ours(cuda, cfg, cam, kt.SCHED_PLAIN)
+        want = want.view(np.uint32)
+        if spp == 1:
+            got, _, _, _ = run_ours(cuda, cfg, cam, kt.SCHED_WAVEFRONT, ctx=ctx)
+            assert np.array_equal(got.view(np.uint32), want)
+        ctx.close()
+        hdr, err = cuda.zeros((n, 4), device="cuda"), cuda.zeros(2, dtype=cuda.int32, device="cuda")
+        b = kt.Batch([(cfg, cam, hdr.data_ptr(), err.data_ptr())])
+        for schedule in (kt.SCHED_PLAIN, kt.SCHED_WAVEFRONT):
+            hdr.zero_()
+            b.set_tuning(schedule, blocks_per_sm=4)
+            b.trace()
+            cuda.cuda.synchronize()
+            assert np.array_equal(hdr.cpu().numpy().view(np.uint32), want), (spp, schedule)
+        b.close()
