@@ -351,8 +351,8 @@ uint64_t kt_batch_rays(const kt_batch* b);
 void kt_batch_destroy(kt_batch* b);
 
 /* ---- trace without any device allocation --------------------------------------------------- */
-/* Largest n_views of one kt_trace_noalloc call.  Its scratch is a 32-bit work counter over all views, in a
- * 256-byte array inside the library's device image. */
+/* Largest n_views of one kt_trace_noalloc call: its cameras travel in a table of the launch's arguments.
+ * Its scratch is a 32-bit work counter over all views, inside the library's device image. */
 #define KT_NOALLOC_MAX_VIEWS 64
 /*
  * No counterpart in the reference.  For callers that cannot allocate device memory where they
@@ -369,7 +369,7 @@ void kt_batch_destroy(kt_batch* b);
  *   err_words  dev uint32[2*n_views], the LUT error word of each view (not cleared here)
  * It runs the wavefront tracer on the current device and stream, reading the LUTs through a
  * model of the texture unit's filter, so its images match kt_trace to the parity tolerance.
- * The first call on a device looks up the scratch array's device address
+ * The first call on a device looks up the scratch word's device address
  * (cudaGetSymbolAddress) with that device current; make that first call before any stream
  * capture.  The address is kept for the life of the process: after a cudaDeviceReset of that
  * device (which unloads the library's device image) do not call this entry point on it again.  Every call shares the scratch: calls that overlap on the GPU race and must be

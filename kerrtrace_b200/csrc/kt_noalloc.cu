@@ -7,10 +7,10 @@
 // in flight.  Such a caller cannot create a kt_context, which allocates its LUT textures and
 // its work counter.  kt_trace_noalloc takes everything from the caller instead — scene
 // configuration, cameras, the two LUTs as plain device arrays, the output buffers — and keeps
-// its only scratch, a work counter, in the file-scope array below.
+// its only scratch, a work counter, in the file-scope word below.
 //
-// The array is part of the library's device image: every GPU that loads the library holds its
-// 256 bytes until the process exits.  Every call shares it and it keeps the last call's
+// The word is part of the library's device image: every GPU that loads the library holds it
+// until the process exits.  Every call shares it and it keeps the last call's
 // count; a call that uses it clears it on its own stream before the trace kernel runs.  Calls that
 // overlap on the GPU (other streams, other host threads on the same device) race on it and must
 // be serialised by the caller.
@@ -29,9 +29,9 @@
 
 namespace ktd {
 
-// Scratch of kt_trace_noalloc: the work counter is its first word.  In host code this name is only a
-// stand-in for the device symbol; its device address comes from cudaGetSymbolAddress.
-static __device__ __align__(256) unsigned int g_noalloc_queue[KT_NOALLOC_MAX_VIEWS];
+// Scratch of kt_trace_noalloc: the work counter, on a 128-byte line of its own.  In host code this name is
+// only a stand-in for the device symbol; its device address comes from cudaGetSymbolAddress.
+static __device__ __align__(128) unsigned int g_noalloc_queue;
 
 struct NoallocViews {
     Camera cam[KT_NOALLOC_MAX_VIEWS];
@@ -111,7 +111,7 @@ static kt_status noalloc_scratch(int device, unsigned** out) {
         const cudaError_t e = cudaGetSymbolAddress(&p, g_noalloc_queue);
         if (e != cudaSuccess) {
             char msg[256];
-            snprintf(msg, sizeof msg, "cudaGetSymbolAddress of the work counters failed: %s", cudaGetErrorString(e));
+            snprintf(msg, sizeof msg, "cudaGetSymbolAddress of the work counter failed: %s", cudaGetErrorString(e));
             return set_error(KT_ERR_CUDA, msg);
         }
         g_noalloc_addr[device] = static_cast<unsigned*>(p);
@@ -130,14 +130,14 @@ extern "C" kt_status kt_trace_noalloc(const kt_config* cfg, const kt_camera* cam
         return set_error(KT_ERR_INVALID_ARG, "kt_trace_noalloc: NULL argument");
     if (n_views == 0 || n_views > KT_NOALLOC_MAX_VIEWS) {
         char msg[160];
-        snprintf(msg, sizeof msg, "kt_trace_noalloc: %u views requested; its scratch holds work counters for 1..%d views",
+        snprintf(msg, sizeof msg, "kt_trace_noalloc: %u views requested; its table of cameras holds 1..%d",
                  n_views, KT_NOALLOC_MAX_VIEWS);
         return set_error(KT_ERR_INVALID_ARG, msg);
     }
     if (cfg->mode != KT_MODE_REF || cfg->precision != KT_PREC_FP32)
         return set_error(KT_ERR_UNSUPPORTED, "kt_trace_noalloc implements the reference semantics in FP32 only");
     if ((uint64_t)cfg->width * cfg->height * n_views >= (1ull << 32))
-        return set_error(KT_ERR_INVALID_ARG, "kt_trace_noalloc: frame too large for the 32-bit work counters");
+        return set_error(KT_ERR_INVALID_ARG, "kt_trace_noalloc: frame too large for the 32-bit work counter");
     Scene sc;
     kt_status st = scene_from_config(cfg, &sc);
     if (st != KT_OK) return st;

@@ -620,8 +620,7 @@ __device__ __forceinline__ void null_renormalise(double* s, double pt, const Sce
     s[5] *= lam;
 }
 
-// The start is the FP32 start (the camera and direction are FP32 data; it runs once per ray in
-// the refill path, where FP64 square roots and divisions would cost as much as the ray's steps).
+// The start is the FP32 start: the camera and direction are FP32 data.
 __device__ __forceinline__ bool ray_start_mixed(RayRun<Mixed>& ry, const Camera& cam, const float dir[3],
                                                 const Scene& sc, bool later_sample) {
     RayRun<float> d;

@@ -307,3 +307,12 @@ def test_disk_tables_equal_the_oracle_restatement(kt, orc, spin, mass, span, siz
     r_out = float(np.float32(p.disk_inner + span))
     got = kt.generate_disk_lut(p, r_out, size)
     assert np.array_equal(got.view(np.uint32), orc.disk_lut(cfg.spin, cfg.mass, r_out, size).view(np.uint32))
+
+
+@pytest.mark.parametrize("n_views", [0, 65, 1000])
+def test_noalloc_names_the_limit_it_refuses_by(kt, n_views):
+    """The number of views is bounded by the table of cameras of a launch (before any device work)."""
+    cfg, cams, word = kt.config_default(), (kt.KtCamera * 65)(), C.c_void_p(64)
+    st = kt.lib().kt_trace_noalloc(C.byref(cfg), cams, n_views, word, word, None, word, word)
+    text = kt.lib().kt_last_error().decode()
+    assert st == kt.KT_ERR_INVALID_ARG and "cameras holds 1..64" in text and "counters" not in text
