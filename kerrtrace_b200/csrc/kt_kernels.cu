@@ -250,8 +250,7 @@ __global__ void __launch_bounds__(MAXT, MINB)
 // side) for one lane of 32, which cost more than the idle lanes it filled.  Against it (trace and
 // post, default tuning; with the later steps in it): 1920x1080 reference 3.58 -> 2.21 ms (trace),
 // 960x540 FP64 5.67 -> 2.42, 1024^2 mixed 2.64 -> 1.09, two frames of 2100x900 at 4 samples 16.0 -> 7.16;
-// 96x64 at 2 samples 0.277 -> 0.080, where a pixel's samples used to run one after the other on one lane; with
-// frozen rays kept to the end (a switch for timing) 183 -> 187.
+// 96x64 at 2 samples 0.277 -> 0.080, where a pixel's samples used to run one after the other on one lane.
 template <class R, int MODE, bool COUNT, int MINB, bool TOGETHER, bool STRIPS>
 __global__ void __launch_bounds__(kWavefrontBlock, MINB)
     trace_wavefront_kernel(const __grid_constant__ Scene sc, const Camera cam, float4* __restrict__ hdr,
@@ -374,9 +373,12 @@ static cudaError_t launch_wave_minb(const Scene& sc, const Camera& cam, float4* 
     // caches; persistent warps drift apart and the FP64 kernel waited for instructions 0.7
     // cycles per issue.  960x540 FP64 3.24 -> 2.99 ms, 1920x1080 6.58 -> 5.75, 400x300 x 3 samples 2.89 ->
     // 2.66; 1920x1080 FP32 2.16-2.36 -> 2.08.  The mixed and the reference trace gain nothing (1.088 ->
-    // 1.097, 2.217 -> 2.227) and stay persistent.
+    // 1.097, 2.217 -> 2.227) and stay persistent, unless frozen rays are kept to the end (a switch for
+    // timing): such a ray is a hundred times as long as the others of its unit, and blocks that come
+    // up as others end fill the SMs better than warps that were dealt units before (1920x1080
+    // 187 -> 152 ms; single lanes refilled from the counter took 183).
     constexpr bool kAllBlocks = MODE == 1 && !std::is_same<R, Mixed>::value;
-    const unsigned grid = kAllBlocks || blocks < resident ? blocks : resident;
+    const unsigned grid = kAllBlocks || sc.keep_frozen || blocks < resident ? blocks : resident;
     if (units > grid * kWarps) {
         e = cudaMemsetAsync(queue, 0, sizeof(unsigned), st);
         if (e != cudaSuccess) return e;

@@ -141,3 +141,17 @@ def test_schedules_agree_as_documented(cuda, mode, prec, spin, radius, inclinati
             cuda.cuda.synchronize()
             assert np.array_equal(hdr.cpu().numpy().view(np.uint32), want), (spp, schedule)
         b.close()
+
+
+@pytest.mark.parametrize("size", [(48, 20), (640, 400)])
+def test_kept_frozen_rays_in_units(cuda, size):
+    """Frozen rays kept to the end of their budget, in launches of one unit per resident warp and of
+    more: the plain schedule's image without them."""
+    cfg, cam = scene(*size)
+    cfg.max_steps = 3000
+    want, _, _, ctx = run_ours(cuda, cfg, cam, kt.SCHED_PLAIN)
+    for bps in (3, 4):
+        ctx.set_tuning(schedule=kt.SCHED_WAVEFRONT, blocks_per_sm=bps, keep_frozen=1)
+        got, _, _, _ = run_ours(cuda, cfg, cam, kt.SCHED_AUTO, ctx=ctx)
+        assert np.array_equal(got.view(np.uint32), want.view(np.uint32))
+    ctx.close()
