@@ -1067,10 +1067,13 @@ __global__ void __launch_bounds__(256) post_weight_sums_kernel(const PostParams 
 }
 
 constexpr size_t kSmemLimit = 200 * 1024;
-// Largest radius of the horizontal pass and the fused post (about 163).
-static bool radius_fits(int R) {
-    return (size_t)32 * ((kTPos + 2 * R) | 1) * 16 + (size_t)(2 * R + 2 + kTPos) * 4 <= kSmemLimit;
-}
+// Largest radius of the horizontal pass and the fused post.  The tiles of line pairs would take radii up to
+// 229 in kSmemLimit; this is the limit that callers know, at which tiles of 32 single lines filled it, and
+// a radius that was refused stays refused.  The vertical pass alone has no such limit: it takes the
+// tiles as far as they go and post_v_wide_kernel beyond.
+constexpr int kMaxRadius = 165;
+static_assert(pair_smem(kMaxRadius) <= kSmemLimit, "the largest radius fits its tile");
+static bool radius_fits(int R) { return R <= kMaxRadius; }
 
 // Lets a kernel be launched with `bytes` of shared memory.  The attribute belongs to the function, not
 // to the launch, so it is always raised to the same limit: with the size of the call at hand, a

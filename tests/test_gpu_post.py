@@ -269,3 +269,42 @@ def test_post_passes_of_two_radii_from_two_threads(cuda):
     assert not failed, (len(failed), failed[0])
     for i in range(2):
         assert cuda.equal(img[i], want[i])
+
+
+@pytest.mark.parametrize("radius,taken", [(165.0, True), (165.5, False), (229.0, False), (230.0, False)])
+def test_largest_radius_of_each_pass(cuda, orc, radius, taken):
+    """The horizontal and the fused pass take radii up to 165; the vertical pass takes all of these, tiled
+    up to 229 and one pixel per thread beyond: the image is the oracle's to one code value."""
+    cfg, _ = workloads.scene("t1")
+    cfg = workloads.scaled(cfg, 40, 90)
+    cfg.bloom_radius = radius
+    R, sigma, _ = _bloom_consts(cfg)
+    w, h = cfg.width, cfg.height
+    hdr = _hdr_input(cuda, cfg, 31)
+    ctx = kt.Context(cfg)
+    bloom = cuda.zeros((w * h, 4), device="cuda")
+    img_s, img_f = (cuda.zeros(w * h, dtype=cuda.int32, device="cuda") for _ in range(2))
+    if taken:
+        ctx.bloom_horizontal(hdr.data_ptr(), bloom.data_ptr())
+        ctx.post_fused(hdr.data_ptr(), img_f.data_ptr())
+    else:
+        for refused in (lambda: ctx.bloom_horizontal(hdr.data_ptr(), bloom.data_ptr()),
+                        lambda: ctx.post_fused(hdr.data_ptr(), img_f.data_ptr())):
+            with pytest.raises(kt.KtError):
+                refused()
+        k = np.exp(-np.arange(-R, R + 1) ** 2 / (2 * sigma ** 2))
+        src = np.zeros((h, w + 2 * R, 4))
+        src[:, R:R + w, :3] = hdr.cpu().numpy().reshape(h, w, 4)[..., :3]
+        src[:, R:R + w, 3] = 1.0
+        b = sum(k[i] * src[:, i:i + w] for i in range(2 * R + 1))
+        bloom[:, :3] = cuda.from_numpy((b[..., :3] / b[..., 3:]).reshape(-1, 3).astype(np.float32)).cuda()
+    ctx.post_process(hdr.data_ptr(), bloom.data_ptr(), img_s.data_ptr())
+    cuda.cuda.synchronize()
+    got = img_s.cpu().numpy().view(np.uint32)
+    if taken:
+        assert np.array_equal(got, img_f.cpu().numpy().view(np.uint32))
+    exp = orc.post(hdr.cpu().numpy(), w, h, R, sigma, cfg.bloom_intensity)
+    d = np.max(np.abs(np.stack([(got >> s) & 255 for s in (16, 8, 0)]).astype(int) -
+                      np.stack([(exp >> s) & 255 for s in (16, 8, 0)]).astype(int)), axis=0)
+    assert d.max() <= 1, np.bincount(d)
+    ctx.close()
