@@ -22,6 +22,9 @@ radius 24, ACES + sRGB): the trace kernel plus the post-processing kernel.
 oracle/_ref) with the launch sequence of src/renderer/mod.rs: trace_kernel, bloom_horizontal,
 post_process, image copy to pinned host memory.
 
+One JSON line on stdout: these, and the main values of the other legs; the whole record, with every
+candidate and sweep, on stderr.
+
 Multi-GPU (torchrun): every rank renders its own frame of the same scene seen from a different
 azimuth (the spacetime is axisymmetric, so every rank has the same work): weak scaling, no
 data-path collective; the time is the max over ranks.
@@ -77,6 +80,32 @@ def parse():
                     help="schedule,block_x,block_y,blocks_per_sm,refill_min,order: this launch shape instead of "
                          "the autotuner's (reproducible profiling)")
     return ap.parse_args()
+
+
+# Legs of a run beside its headline.
+LEGS = ("autotune", "retirement", "precision", "adjoint", "batch", "pareto", "sequence", "c3")
+
+
+def headline(line: dict) -> dict:
+    """The line for stdout, a few KB: the headline keys whole, and of each leg the plain values of its
+    top level and of its groups (no lists, nothing deeper, no clocks and launch shapes).  The whole
+    record, tables of candidates and sweeps included (about 33 KB), goes to stderr."""
+    def plain(v):
+        return isinstance(v, (bool, int, float, str)) or v is None
+
+    def values(group):
+        return {k: v for k, v in group.items() if plain(v)}
+
+    out = {k: v for k, v in line.items() if k not in LEGS}
+    for name in LEGS:
+        if name not in line:
+            continue
+        leg = values(line[name])
+        for k, v in line[name].items():
+            if isinstance(v, dict) and k not in ("clocks", "tuning", "shapes") and values(v):
+                leg[k] = values(v)
+        out[name] = leg
+    return out
 
 
 class ClockSampler:
@@ -906,7 +935,8 @@ def run_ours(args, rank, world, local):
     if rank == 0 and world == 1 and not args.no_cpu_baseline:
         line["cpu_baseline"] = cpu_baseline(cfg, cam, args.cpu_seconds)
     if rank == 0:
-        print(json.dumps(line), flush=True)
+        print(json.dumps(line), file=sys.stderr, flush=True)
+        print(json.dumps(headline(line)), flush=True)
     ctx.close()
 
 

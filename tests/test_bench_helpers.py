@@ -40,3 +40,24 @@ def test_both_arms_describe_the_same_workload(kt, orc):
         c_ref, cam_ref = bench.rank_camera(workloads, "c2", 0, 1, size, host=orc.Host())
         assert bench.workload_label("c2", c_lib) == bench.workload_label("c2", c_ref)
         assert bytes(c_lib) == bytes(c_ref) and bytes(cam_lib) == bytes(cam_ref)
+
+
+def test_headline_line_keeps_its_keys_and_stays_short():
+    """The stdout line: headline keys whole, of each leg the plain values only, and a few KB however many
+    rows the tables of a leg hold."""
+    import json
+    rows = [{"ms": 1.0 + i, "tuning": {"schedule": 0}} for i in range(500)]
+    line = {"metric": "m", "value": 1.5, "config": {"tuning": {"block_x": 8}, "l2": "flushed"},
+            "e2e": {"value": 1.0, "h2d_bytes_per_step": 52}, "roofline": {"frac": 0.5, "work": {"rays": 1}},
+            "clocks": {"sm_mhz": 1965.0, "reasons": []}, "gpu_launches": 30,
+            "autotune": {"best": {"block_x": 8}, "best_ms": 2.0, "top": rows, "candidates": 500},
+            "precision": {"fp64": {"mrays_s": 3.0, "tuning": {"a": 1}, "err": {"p99": 1.0}}, "clocks": {"sm_mhz": 1.0}},
+            "pareto": {"scenes": {"c2": {"size": "1x1", "points": rows}}, "tolerances": [1e-5] * 500},
+            "c3": {"size": 4096, "runs": rows}, "batch": {"tuner": rows, "batched_launch": {"mrays_s": 1.0}}}
+    out = bench.headline(line)
+    for k in ("metric", "value", "config", "e2e", "roofline", "clocks", "gpu_launches"):
+        assert out[k] == line[k]
+    assert out["autotune"] == {"best_ms": 2.0, "candidates": 500, "best": {"block_x": 8}}
+    assert out["precision"] == {"fp64": {"mrays_s": 3.0}} and out["c3"] == {"size": 4096}
+    assert out["batch"] == {"batched_launch": {"mrays_s": 1.0}} and out["pareto"] == {}
+    assert len(json.dumps(out)) < 2000
