@@ -66,6 +66,10 @@ template <> struct Ops<float> {
 // of a subnormal and of an infinity is NaN too; its arguments here, r^2 + a^2 and r^4 + a^2 y^2,
 // take such values only where r itself is NaN already (r = r2 rsqrt(r2), 0 x inf).  The square
 // root keeps 0 and infinity.
+//
+// With the operators and with these: c2 view in FP64, 960x540 3.43 -> 2.73 ms (plain 32x4, 3 per SM) and
+// 3.48 -> 2.85 (wavefront), 1920x1080 6.65 -> 5.58 and 6.79 -> 5.73; recording forward of 256x256 636 ->
+// 522 us.
 template <> struct Ops<double> {
     static __device__ __forceinline__ double rsq(double x) { return rsqrt(x); }
     static __device__ __forceinline__ double inv(double b) {

@@ -97,8 +97,8 @@ __device__ __forceinline__ void dense_weights(R t, R h, R w[8]) {
 //   Hk = M k / r,  Hk_r = M k^2 (3w - 1) / r^2,  Hk_rr = 2 M k^3 (3w^2 - 12w + 1) / r^3
 // (and their a^2 y^2-derivatives in units of r^4, so that no high power of r under- or overflows in
 // float).  About 210 operations; the dual-number evaluation of the right-hand side in three
-// directions that it replaces took 700 and spilled in double.  Loss gradient at 512x512: FP32 1.18 ->
-// 0.48 ms, FP64 1.94 -> 0.95 ms, FP64 over FP32 records 2.29 -> 1.15 ms.
+// directions that it replaces took 700 and spilled in double.  Backward call of a fit at 512x512, with the
+// steps below: FP32 1.36 -> 0.50 ms, FP64 2.32 -> 1.03, FP64 over FP32 records 2.84 -> 1.31.
 template <class R>
 __device__ __forceinline__ void rhs_vjp(const R* Y, const R* l, R pt, R a, R aa, R M, R* out, R& da, R& dpt) {
     using O = Ops<R>;
@@ -160,8 +160,8 @@ __device__ __forceinline__ void rhs_vjp(const R* Y, const R* l, R pt, R a, R aa,
 
 // The float product as a call (arguments and results in registers): seven inlined copies made the reverse
 // step 70 KB of straight code, and with two warps per scheduler a quarter of the time went to
-// instruction fetches (512x512: 444 -> 414 us).  In double the copies are the faster form (the
-// call spills around its 24 registers of arguments: 669 -> 742 us at 256x256).
+// instruction fetches (the call takes 7% off the backward at 512x512).  In double the copies are the
+// faster form (the call spills around its 24 registers of arguments: 11% more at 256x256).
 struct Vec6 {
     float v[6];
 };
@@ -455,9 +455,10 @@ __device__ __forceinline__ R rk_a(int m, int j) {
 
 // ---- forward: record / replay ----------------------------------------------------------------
 // Resident 128-thread blocks per SM asked of the compiler: four in FP32 (128 registers at most), three in
-// FP64 (168; with four the kernel spills 380 B: 512x512 1.14 ms against 1.03).  A warp takes an 8x4
-// patch of the frame, whose rays have more equal lengths than a row's 32 (512x512: FP32 437 -> 391
-// us with the host's tables, FP64 1.39 -> 1.14 ms).
+// FP64 (168; with four the kernel spills 380 B and is 10% slower).  A warp takes an 8x4
+// patch of the frame, whose rays have more equal lengths than a row's 32 (12% in FP32, 18% in FP64 at
+// 512x512).  Forward call there, host tables included, with both and the packed stage sums: FP32 452 -> 376
+// us, FP64 1.73 -> 1.10 ms.
 // RR: arithmetic type of the records (R, or float records replayed in double arithmetic).
 template <class R, bool REPLAY, bool STRIPS, class RR = R>
 __global__ void __launch_bounds__(128, sizeof(R) == 8 ? 3 : 4) diff_forward_kernel(const Scene sc, const Camera cam, const CameraD camd,
@@ -685,7 +686,7 @@ __device__ __forceinline__ void replay_segment_start(const DiffRay& rr, const Di
         sweep_segment<R, RR>(seg_at<RR>(rec, si), ry0.pt, ry0.kt, a, aa, M, sc, dl, k, k7, s, tau);
 }
 
-// Resident 128-thread blocks per SM asked of the compiler for the adjoint kernel: two (193 registers
+// Resident 128-thread blocks per SM asked of the compiler for the adjoint kernel: two (183 registers
 // in FP32, no spills).
 template <class R> struct BackMinBlocks { static constexpr int v = 2; };
 template <> struct BackMinBlocks<double> { static constexpr int v = 2; };
@@ -756,7 +757,7 @@ __global__ void __launch_bounds__(128, BackMinBlocks<R>::v) diff_backward_kernel
                 const unsigned hits = sg->hits;
                 // the last segment ends with the ray's last shaded crossing: the transmittance behind it
                 // has no use, and its root and shading, at a different step of each lane, are left out
-                // (512x512: FP32 479 -> 444 us, FP64 955 -> 816)
+                // (7% of the call at 512x512 in FP32, 15% in FP64)
                 const int n = first ? 32 - __clz((int)hits) : sg->n;
                 const int last_hit = first ? n - 1 : -1;
                 first = false;

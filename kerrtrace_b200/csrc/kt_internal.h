@@ -117,9 +117,10 @@ inline bool take_strips(int W, int H, unsigned patch_units, unsigned warps) {
 // while that one drains, and call wait_for_stream() before the rest.  wait_for_stream() returns
 // when everything ahead in the stream has ended and its writes are visible, so every kernel launched
 // this way keeps the stream's order; it does nothing in a kernel launched the plain way.  What it
-// saves is the gap between two launches, about 2 us each: fused post of 96x64 14.4 -> 9.1 us,
-// 960x540 20.7 -> 16.5, 3840x2160 168 -> 164 (two launches); a 96x64 frame with its post 83.9 ->
-// 77.2 (three).
+// saves is the gap between two launches, about 2 us each (back to back, launched the plain way and this
+// way): fused post of 96x64 15.4 -> 11.5 us, 960x540 20.5 -> 16.1, 1920x1080 45.1 -> 41.1, 3840x2160
+// 162.9 -> 159.2 (two launches); the two tables of 4096 rows 11.3 -> 7.1 (two); a 96x64 frame of 2
+// samples with its post 117.7 -> 110 (three).
 template <class F, class... A>
 cudaError_t launch_early(F kernel, dim3 grid, int block, size_t smem, cudaStream_t st, A... args) {
     cudaLaunchAttribute at = {};

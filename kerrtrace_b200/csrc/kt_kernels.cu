@@ -249,8 +249,8 @@ __global__ void __launch_bounds__(MAXT, MINB)
 // rays ended: each refill ran the start-up code (ray set-up, first tolerance, first right-hand
 // side) for one lane of 32, which cost more than the idle lanes it filled.  Against it (trace and
 // post, default tuning; with the later steps in it): 1920x1080 reference 3.58 -> 2.21 ms (trace),
-// 960x540 FP64 5.67 -> 2.42, 1024^2 mixed 2.64 -> 1.09, two frames of 2100x900 at 4 samples 16.0 -> 7.16;
-// 96x64 at 2 samples 0.277 -> 0.080, where a pixel's samples used to run one after the other on one lane.
+// 960x540 FP64 6.27 -> 2.99, 1024^2 mixed 2.62 -> 1.09, two frames of 2100x900 at 4 samples 15.6 -> 7.13;
+// 96x64 at 2 samples 0.279 -> 0.075, where a pixel's samples used to run one after the other on one lane.
 template <class R, int MODE, bool COUNT, int MINB, bool TOGETHER, bool STRIPS>
 __global__ void __launch_bounds__(kWavefrontBlock, MINB)
     trace_wavefront_kernel(const __grid_constant__ Scene sc, const Camera cam, float4* __restrict__ hdr,
@@ -655,11 +655,12 @@ __device__ __forceinline__ float4 bloom_source(float4 c, const PostParams& pp) {
 // plain multiply-adds of an earlier form competed with them for slots and kept the pipe 37% busy.
 // 64 x 32-pixel tiles of 128 threads: 43 KB and 5 blocks per SM at R = 24, 7 blocks per SM and
 // frame at 1920x1080 (1020 blocks: a 128-wide tile would leave some SMs 4 and some 3).  Both passes
-// back to back (fused), their launches overlapped (launch_early): 1920x1080 R = 24 66.4 -> 40.8 us,
-// 3840x2160 213 -> 159 us, 2100x900 R = 48 118 -> 64.4 us, 960x540 30.9 -> 16.2 us.  Without the
-// overlap 1920x1080 takes 45.3 us, without the blur as well 31, without the staging 41: what is left
+// back to back (fused), their launches overlapped (launch_early): 1920x1080 R = 24 66.4 -> 41.1 us,
+// 3840x2160 213 -> 159 us, 2100x900 R = 48 118 -> 66.4 us, 960x540 30.9 -> 16.1 us.  Without the
+// overlap 1920x1080 takes 45.1 us, without the blur as well 31, without the staging 41: what is left
 // beside the multiply-adds (18 us) is each block's chain of loads, tone map and stores with 16 to
-// 20 warps per SM to cover it.
+// 20 warps per SM to cover it (FMA pipe 41 and 45% active, issue 36 and 45%; 3.0 and 2.0 cycles of
+// waiting for loads per issue).
 constexpr int kBJ = 8, kTPairs = 16, kTPos = 64, kTThreads = kTPairs * (kTPos / kBJ);
 constexpr int kTWarps = kTThreads / 32;
 

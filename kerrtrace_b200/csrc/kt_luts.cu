@@ -33,7 +33,7 @@ __device__ float cmf_lobe_d(float x, float alpha, float mu, float s1, float s2) 
 // per row and channel.  With one thread per row doing all of it (7 exponentials of the matching
 // functions per term), back to back: 4096 rows x 35 wavelengths 30.9 us, now 7.3; 16384 x 341 252 us,
 // now 46; 100 x 1134 854 us, now 82.  Both table kernels come up under the one ahead and wait for it
-// only before they store (launch_early): the two tables of 4096 rows, in turn, 10.6 -> 7.4 us.
+// only before they store (launch_early): the two tables of 4096 rows, in turn, 11.3 -> 7.1 us.
 constexpr int kRows = 16, kChunk = 64, kLutThreads = 128;
 __global__ void __launch_bounds__(kLutThreads) blackbody_lut_kernel(uint32_t size, float max_temp, float wl_start,
                                                                     int n_lambda, float wl_step,
